@@ -391,8 +391,8 @@ PRAMAAN_API int pramaan_launch_pdhg_iteration(float* h_x, float* h_y, const floa
  * graph, and hosts that own the device memory pool.  All pointers are device
  * pointers owned by the caller (row_ptr[m+1], col_idx[nnz], values[nnz], x[n],
  * y[m]); the work is queued on `stream` (a cudaStream_t, NULL for the legacy
- * default stream) and the call returns without waiting.  Partial sums of rows
- * that cross 2048-entry tiles go to a 512 KiB scratch array compiled into the
+ * default stream) and the call returns without waiting.  Partial sums of very
+ * long rows (from 512 entries on) go to a 512 KiB scratch array compiled into the
  * library (a file-scope __device__ array, held by every GPU that loads the
  * library until exit), which limits nnz to 134,217,728; larger inputs are
  * rejected with PRAMAAN_ERR_INVALID_ARGUMENT.  Every call shares that array:

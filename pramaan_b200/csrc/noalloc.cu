@@ -10,19 +10,38 @@
 // the caller's stream and allocates nothing: no cudaMalloc, no cudaFree, no
 // allocating library routine.
 //
-// The product is the nnz-balanced ("merge-path") scheme of the library's main
-// SpMV, restated for a plain CSR that has not been converted to the tiled
-// format: each block takes T = 2048 consecutive entries, finds its rows by
-// binary search in row_ptr, and combines partial sums with a segmented block
-// scan.  A row that crosses tile boundaries leaves one partial per tile in a
-// scratch array; a second kernel adds each crossing row's partials in tile
-// order.  That scratch is the file-scope array below: every GPU that loads
-// the library holds it (512 KiB) until the process exits, it limits one call
-// to kNoAllocMaxTiles tiles (nnz <= 134,217,728), and every call shares it,
-// so calls that overlap on the GPU (on different streams) race; calls on one
-// stream are ordered.  Every slot a call reads is written earlier in the same
-// call, so nothing needs clearing between calls.
+// The product splits the non-zeros evenly over warps: warp k owns the rows
+// that start in entries [k T, (k + 1) T) and streams their entries in tiles of
+// 256 (coalesced loads, 8 gathers of x in flight per lane, products through
+// shared memory, then the rows of the tile summed by 1 to 8 lanes each, or by
+// the whole warp where a row is long).  Owning whole rows leaves nothing to
+// combine between warps, except for giant rows (more than 2 T entries): those
+// are cut at the range boundaries, every range sums its piece into the scratch
+// array below, and the pieces of a row are added in a fixed order afterwards:
+// by the same launch when the whole product fits one thread-block cluster
+// (nnz <= 16,384), else by a second, dependent one.  The scratch is the
+// file-scope array below: every GPU that loads the library holds it (512 KiB)
+// until the process exits, one call is limited to nnz <= 134,217,728, and
+// every call shares it, so calls that overlap on the GPU (on different
+// streams) race; calls on one stream are ordered.  Every slot a call reads is
+// written earlier in the same call, so nothing needs clearing between calls.
+//
+// What bounds it: the gathers.  B200 serves random 4-byte gathers at about one
+// sector per SM per clock (ceiling.cu), 14 us for 4 M entries and 97 us for
+// 27 M, and the stream's own sectors share that path.  Small products are
+// bound by the chain search - row pointers - entries - gather - sums, five L2
+// round trips.  Measured per call in a captured graph (before: tiles of 2,048
+// entries per block, serial searches by one thread, a completion kernel that
+// searched again):
+//   1,000 x 3,000, 12 K entries              5.3 us
+//   200,000 x 500,000, 4 M, uniform         25.7 us   (58.8 us of kernel time)
+//   500,000 x 1,250,000, 27 M, power law     136 us   (238 us of kernel time)
+//   the same size, 25.6 M, banded             61 us   (0.53 of the HBM copy rate)
+// Tiles of 512 entries (64 registers, 32 warps per SM instead of 48) cost
+// 65 us on the banded and 18 against 16.5 us on a 1 M-entry product.
+#include <algorithm>
 #include <atomic>
+#include <climits>
 #include <mutex>
 #include <string>
 
@@ -31,16 +50,20 @@
 namespace pb {
 namespace {
 
-constexpr int kNaBlock = 256;
-constexpr int kNaIpt = 8;
-constexpr int kNaTile = kNaBlock * kNaIpt;           // 2048 entries per tile
-constexpr int kNoAllocMaxTiles = 65536;              // nnz <= 65536 * 2048
-constexpr int kNaRpCap = kNaTile + 8;                // row_ptr slice capacity
+constexpr int kNaWarps = 8;                          // warps per block
+constexpr int kNaTile = 256;                         // entries per warp tile
+constexpr int kNaChunks = kNaTile / 128;             // 16-byte loads per lane and array
+constexpr int kNoAllocMaxNnz = 134217728;
+constexpr int kNaSlots = 3;                          // scratch words per range
+constexpr int kNaMaxRanges = 32768;
+constexpr int kNaClusterBlocks = 8;                  // largest portable cluster
+constexpr int kNaLaneRow = 32;                       // entries of a row one lane sums at most
+constexpr int kNaLocalSpan = 16384;                  // columns: a tile within this span gathers through L1
 
-// Cross-tile partials: slot 2t holds the piece of the row that continues into
-// tile t from earlier tiles (its last or a middle piece), slot 2t+1 the first
-// piece of the row that begins in tile t and continues past it.
-__device__ __align__(256) float g_noalloc_carry[2 * kNoAllocMaxTiles];
+// Scratch: range k has words 3k (its piece of a giant row that began earlier),
+// 3k + 1 (its piece of a giant row that begins here) and 3k + 2 (that row, or -1).
+__device__ __align__(256) float g_noalloc_carry[131072];
+static_assert(kNaSlots * kNaMaxRanges <= 131072, "scratch words");
 
 // Per device ordinal: the array's device address and the SM count, looked up
 // once with that device current.  The address belongs to the runtime's primary
@@ -49,141 +72,323 @@ std::atomic<float*> g_carry_addr[64];
 std::atomic<int> g_sm_count[64];
 std::mutex g_setup_mutex;
 
-// row_ptr read with the padding convention: row m+1 ends at the padded end.
-__device__ __forceinline__ int rp_at(const int* __restrict__ row_ptr, int m, int nnz_pad, int r) {
-    return r <= m ? __ldg(row_ptr + r) : nnz_pad;
+struct NaArgs {
+    const int* __restrict__ row_ptr;
+    const int* __restrict__ col;
+    const float* __restrict__ val;
+    const float* __restrict__ x;
+    float* __restrict__ y;
+    float* carry;
+    int m, n, nnz, T, ranges;
+};
+
+__device__ __forceinline__ int4 ld_stream(const int4* p) {
+    int4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+    float4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
 }
 
-// max r in [0, m] with row_ptr[r] <= q
-__device__ int row_holding(const int* __restrict__ row_ptr, int m, long long q) {
-    int lo = 0, hi = m;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(row_ptr + mid) <= q) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-__global__ void __launch_bounds__(kNaBlock)
-    noalloc_spmv_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col,
-                        const float* __restrict__ val, int m, int n, int nnz,
-                        const float* __restrict__ x, float* __restrict__ y,
-                        float* __restrict__ carry) {
-    __shared__ int s_rp[kNaRpCap];
-    __shared__ int s_lohi[2];
-    __shared__ int s_wrow[kNaBlock / 32];
-    __shared__ float s_wval[kNaBlock / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nt = (nnz + kNaTile - 1) / kNaTile;
-    const int nnz_pad = nt * kNaTile;
-    const unsigned last_col = static_cast<unsigned>(n - 1);
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int tile_base = t * kNaTile, tile_end = tile_base + kNaTile;
-        if (tid == 0) {
-            s_lohi[0] = t == 0 ? 0 : row_holding(row_ptr, m, tile_base);
-            s_lohi[1] = t == nt - 1 ? m : row_holding(row_ptr, m, tile_end);
-        }
-        __syncthreads();
-        const int r_lo = s_lohi[0], r_hi = s_lohi[1];
-        const int cnt = r_hi - r_lo + 2;
-        const bool in_smem = cnt >= 1 && cnt <= kNaRpCap;
-        if (in_smem)
-            for (int j = tid; j < cnt; j += kNaBlock) s_rp[j] = rp_at(row_ptr, m, nnz_pad, r_lo + j);
-        __syncthreads();
-        // Rows outside the loaded slice (reachable only when row_ptr is not
-        // nondecreasing) are read from global memory, never past s_rp.
-        auto rp = [&](int r) {
-            const int j = r - r_lo;
-            return (in_smem && j >= 0 && j < cnt) ? s_rp[j] : rp_at(row_ptr, m, nnz_pad, r);
-        };
-
-        const int k0 = tile_base + tid * kNaIpt, k1 = k0 + kNaIpt;
-        float p[kNaIpt];
+// First row r in [0, m] with row_ptr[r] >= lo_target (r_lo) and hi_target
+// (r_hi), m when there is none, by the whole warp: 32 probes per step, so
+// about log32(m) dependent loads.  Each step shrinks its interval whatever
+// row_ptr holds.
+__device__ __forceinline__ void first_rows(const int* __restrict__ rp, int m, int lo_target, int hi_target, int lane,
+                                           int& r_lo, int& r_hi) {
+    int lo[2] = {0, 0}, width[2] = {m, m};   // the answers lie in [lo, lo + width]
+    const int target[2] = {lo_target, hi_target};
+    while ((width[0] | width[1]) > 0) {
+        int stride[2], probe[2];
 #pragma unroll
-        for (int j = 0; j < kNaIpt; ++j) {
-            const int k = k0 + j;
-            if (k < nnz) {
-                unsigned c = static_cast<unsigned>(__ldg(col + k));
-                c = c < last_col ? c : last_col;   // malformed input never reads out of bounds
-                p[j] = __ldg(val + k) * __ldg(x + c);
-            } else {
-                p[j] = 0.0f;
+        for (int q = 0; q < 2; ++q) {
+            stride[q] = (width[q] >> 5) + 1;
+            const int at = lane * stride[q];
+            probe[q] = at < width[q] ? __ldg(rp + lo[q] + at) : INT_MAX;   // beyond the interval: at or above
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const unsigned yes = __ballot_sync(0xffffffffu, probe[q] >= target[q]);
+            if (width[q] == 0) continue;
+            const int j = yes ? __ffs(int(yes)) - 1 : 32;   // first probe at or above the target
+            const int end = min(j * stride[q], width[q]);
+            const int begin = j > 0 ? (j - 1) * stride[q] + 1 : 0;
+            lo[q] += begin;
+            width[q] = end - begin;
+        }
+    }
+    r_lo = lo[0];
+    r_hi = lo[1];
+}
+
+__device__ __forceinline__ float warp_total(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Sum of entries [b, e) by the whole warp (a piece of a giant row).
+__device__ __forceinline__ float piece_sum(const NaArgs& a, int b, int e, unsigned last_col, int lane) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int k = b + lane; k < e; k += 128) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int q = k + 32 * u;
+            if (q < e) {
+                const unsigned c = min(static_cast<unsigned>(__ldg(a.col + q)), last_col);
+                s[u] = fmaf(__ldg(a.val + q), __ldcg(a.x + c), s[u]);
             }
         }
-        // first row whose end lies beyond k0 (thread 0 of tile 0 also owns rows ending at 0)
-        int r;
-        {
-            int lo = r_lo, hi = r_hi;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (rp(mid + 1) > k0) hi = mid; else lo = mid + 1;
+    }
+    return warp_total((s[0] + s[1]) + (s[2] + s[3]));
+}
+
+// Products of entries [base, base + kNaTile) into p.  kVec: col and val are
+// 16-byte aligned, so lane l takes 4 consecutive entries per load.  kEdge: the
+// tile holds entries outside [e0, e1) (other ranges' or none), which cost no
+// gather; the others skip those tests.
+template <bool kVec, bool kEdge>
+__device__ __forceinline__ void tile_products(const NaArgs& a, int base, int e0, int e1, unsigned last_col, int lane,
+                                              float* __restrict__ p) {
+    unsigned c[4 * kNaChunks];
+    float v[4 * kNaChunks];
+    bool own[4 * kNaChunks];
+#pragma unroll
+    for (int u = 0; u < kNaChunks; ++u) {
+        if (kVec && (!kEdge || base + u * 128 + lane * 4 + 3 < a.nnz)) {
+            const int q = base + u * 128 + lane * 4;
+            const int4 c4 = ld_stream(reinterpret_cast<const int4*>(a.col + q));
+            const float4 v4 = ld_stream(reinterpret_cast<const float4*>(a.val + q));
+            c[4 * u] = c4.x; c[4 * u + 1] = c4.y; c[4 * u + 2] = c4.z; c[4 * u + 3] = c4.w;
+            v[4 * u] = v4.x; v[4 * u + 1] = v4.y; v[4 * u + 2] = v4.z; v[4 * u + 3] = v4.w;
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int q = kVec ? base + u * 128 + lane * 4 + t : base + (4 * u + t) * 32 + lane;
+                const bool in = !kEdge || q < a.nnz;
+                c[4 * u + t] = in ? static_cast<unsigned>(__ldg(a.col + q)) : 0u;
+                v[4 * u + t] = in ? __ldg(a.val + q) : 0.f;
             }
-            r = (t == 0 && tid == 0) ? 0 : lo;
         }
-        float acc = 0.0f, head_acc = 0.0f;
-        int nemit = 0, head_row = -1;
-        auto finish_row = [&](int row) {
-            if (nemit == 0 && rp(row) < k0) { head_row = row; head_acc = acc; }
-            else y[row] = acc;
-            ++nemit;
-            acc = 0.0f;
-        };
+    }
 #pragma unroll
-        for (int j = 0; j < kNaIpt; ++j) {
-            while (r < m && r <= r_hi && rp(r + 1) <= k0 + j) { finish_row(r); ++r; }
-            acc += p[j];
-        }
-        while (r < m && r <= r_hi && rp(r + 1) <= k1) { finish_row(r); ++r; }
-
-        // segmented block scan of (tail row, tail partial)
-        int krow = r;
-        float kval = acc;
+    for (int k = 0; k < 4 * kNaChunks; ++k) {
+        const int q = kVec ? base + (k / 4) * 128 + lane * 4 + k % 4 : base + k * 32 + lane;
+        own[k] = !kEdge || (q >= e0 && q < e1);
+        c[k] = min(c[k], last_col);   // malformed input never reads out of bounds
+    }
+    // Local columns (banded, multi-period; judged by one column per lane):
+    // neighbouring rows share lines in L1.  Spread ones would only evict what
+    // other warps wait for.
+    const bool local = __reduce_max_sync(0xffffffffu, c[0]) - __reduce_min_sync(0xffffffffu, c[0]) < kNaLocalSpan;
+    float g[4 * kNaChunks];
+    if (local) {
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int ro = __shfl_up_sync(0xffffffffu, krow, d);
-            const float vo = __shfl_up_sync(0xffffffffu, kval, d);
-            if (lane >= d && ro == krow) kval += vo;
+        for (int k = 0; k < 4 * kNaChunks; ++k) g[k] = own[k] ? __ldca(a.x + c[k]) : 0.f;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4 * kNaChunks; ++k) g[k] = own[k] ? __ldcg(a.x + c[k]) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kNaChunks; ++u) {
+        if (kVec) {
+            reinterpret_cast<float4*>(p)[u * 32 + lane] =
+                make_float4(v[4 * u] * g[4 * u], v[4 * u + 1] * g[4 * u + 1], v[4 * u + 2] * g[4 * u + 2],
+                            v[4 * u + 3] * g[4 * u + 3]);
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) p[(4 * u + t) * 32 + lane] = v[4 * u + t] * g[4 * u + t];
         }
-        if (lane == 31) { s_wrow[warp] = krow; s_wval[warp] = kval; }
-        __syncthreads();
-        int prow = -1;
-        float pval = 0.0f;
-        for (int w = 0; w < warp; ++w) {
-            if (s_wrow[w] == prow) pval += s_wval[w]; else { prow = s_wrow[w]; pval = s_wval[w]; }
-        }
-        if (krow == prow) kval += pval;
-        int erow = __shfl_up_sync(0xffffffffu, krow, 1);
-        float eval = __shfl_up_sync(0xffffffffu, kval, 1);
-        if (lane == 0) { erow = prow; eval = pval; }
-
-        if (head_row >= 0) {
-            const float tot = head_acc + (erow == head_row ? eval : 0.0f);
-            if (rp(head_row) >= tile_base) y[head_row] = tot;
-            else carry[2 * t] = tot;                 // last piece of a crossing row
-        }
-        if (tid == kNaBlock - 1 && krow < m && rp(krow) < tile_end && rp(krow + 1) > tile_end) {
-            carry[2 * t + (rp(krow) >= tile_base ? 1 : 0)] = kval;   // first or middle piece
-        }
-        __syncthreads();
     }
 }
 
-// For every tile where a crossing row begins: add the row's pieces in tile order.
-__global__ void noalloc_fixup_kernel(const int* __restrict__ row_ptr, int m, int nnz,
-                                     const float* __restrict__ carry, float* __restrict__ y) {
-    const int nt = (nnz + kNaTile - 1) / kNaTile;
-    const int nnz_pad = nt * kNaTile;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt - 1; t += gridDim.x * blockDim.x) {
-        const long long tile_base = t * (long long)kNaTile, tile_end = tile_base + kNaTile;
-        const int R = row_holding(row_ptr, m, tile_end - 1);
-        if (R >= m) continue;
-        const int start = rp_at(row_ptr, m, nnz_pad, R), end = rp_at(row_ptr, m, nnz_pad, R + 1);
-        if (start < tile_base || end <= tile_end) continue;
-        const int t1 = (end - 1) / kNaTile;
-        float sum = carry[2 * t + 1];
-        for (int tt = t + 1; tt <= t1; ++tt) sum += carry[2 * tt];
-        y[R] = sum;
+// Sum of p[from, to) for each lane's own [from, to); `rows` lanes at most hold
+// a non-empty one, the lowest ones.  1 << kLog lanes share a row: few long
+// rows use the whole warp, many short ones a lane each; a row that would take
+// a lane more than kNaLaneRow steps is summed by the whole warp.
+template <int kLog>
+__device__ __forceinline__ float row_sums(const float* __restrict__ p, int from, int to, int lane) {
+    constexpr int G = 1 << kLog;
+    const int f = kLog ? __shfl_sync(0xffffffffu, from, lane >> kLog) : from;
+    const int t = kLog ? __shfl_sync(0xffffffffu, to, lane >> kLog) : to;
+    const bool mine = t - f <= kNaLaneRow * G;
+    const int end = mine ? t : f;
+    const int longest = __reduce_max_sync(0xffffffffu, end - f);
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
+    const int first = f + (lane & (G - 1));
+    for (int q = 0; q < longest; q += 4 * G) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = first + q + u * G;
+            if (k < end) part[u] += p[k];
+        }
     }
+    float sum = (part[0] + part[1]) + (part[2] + part[3]);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (kLog) sum = __shfl_sync(0xffffffffu, sum, (lane << kLog) & 31);
+    unsigned wide = __ballot_sync(0xffffffffu, to - from > kNaLaneRow * G);
+    while (wide) {
+        const int src = __ffs(int(wide)) - 1;
+        wide &= wide - 1;
+        const int wf = __shfl_sync(0xffffffffu, from, src), wt = __shfl_sync(0xffffffffu, to, src);
+        float w = 0.f;
+        for (int q = wf + lane; q < wt; q += 32) w += p[q];
+        w = warp_total(w);
+        if (lane == src) sum = w;
+    }
+    return sum;
+}
+
+// One range by one warp.
+template <bool kVec>
+__device__ __forceinline__ void range_product(const NaArgs& a, int k, int lane, float* __restrict__ p) {
+    const unsigned last_col = static_cast<unsigned>(a.n - 1);
+    const bool last = k == a.ranges - 1;
+    const int lo = k * a.T, hi = last ? a.nnz : lo + a.T;
+    int r, r1;
+    first_rows(a.row_ptr, a.m, lo, hi, lane, r, r1);
+    if (last) r1 = a.m;   // with the empty rows after the last entry
+    auto rp = [&](int i) { return min(max(__ldg(a.row_ptr + i), 0), a.nnz); };
+    const int e0 = r1 > r ? rp(r) : 0;
+    int e1 = r1 > r ? rp(r1) : 0;
+    // ---- pieces of giant rows ----
+    const int kGiant = 2 * a.T;
+    if (r > 0) {
+        const int s = rp(r - 1), e = r1 > r ? e0 : rp(r);
+        if (e > lo && e - s > kGiant) {
+            const float t = piece_sum(a, lo, min(e, hi), last_col, lane);
+            if (lane == 0) a.carry[kNaSlots * k] = t;
+        }
+    }
+    int giant = -1;
+    if (r1 > r) {
+        const int s = rp(r1 - 1);
+        if (e1 - s > kGiant) {
+            giant = --r1;
+            const float t = piece_sum(a, s, min(e1, hi), last_col, lane);
+            if (lane == 0) a.carry[kNaSlots * k + 1] = t;
+            e1 = s;
+        }
+    }
+    if (lane == 0) a.carry[kNaSlots * k + 2] = __int_as_float(giant);
+
+    // ---- the other rows, tile by tile ----
+    float open = 0.f;   // partial sum of row r, begun in an earlier tile
+    for (int base = e0 & ~3; base < e1; base += kNaTile) {
+        const int lim = base + kNaTile;
+        // the row pointers of the next 32 rows travel with the tile's entries
+        int s = r + lane <= r1 ? rp(r + lane) : INT_MAX;
+        int s_next = r + 32 <= r1 ? rp(r + 32) : INT_MAX;
+        if (base >= e0 && lim <= e1) tile_products<kVec, false>(a, base, e0, e1, last_col, lane, p);
+        else tile_products<kVec, true>(a, base, e0, e1, last_col, lane, p);
+        __syncwarp();
+        while (true) {
+            int e = __shfl_down_sync(0xffffffffu, s, 1);
+            if (lane == 31) e = s_next;
+            const bool started = r + lane < r1 && s < lim;
+            const bool done = started && e <= lim;
+            const unsigned started_m = __ballot_sync(0xffffffffu, started);
+            const int nd = __popc(__ballot_sync(0xffffffffu, done));
+            // the next rows' pointers, before the sums of these
+            int s2 = INT_MAX, s2_next = INT_MAX;
+            if (nd == 32) {
+                s2 = r + 32 + lane <= r1 ? rp(r + 32 + lane) : INT_MAX;
+                s2_next = r + 64 <= r1 ? rp(r + 64) : INT_MAX;
+            }
+            const int from = started ? max(s, base) - base : 0;
+            const int to = started ? min(e, lim) - base : 0;
+            const int rows = __popc(started_m);
+            float sum = rows > 16 ? row_sums<0>(p, from, to, lane)
+                        : rows > 8 ? row_sums<1>(p, from, to, lane)
+                        : rows > 4 ? row_sums<2>(p, from, to, lane) : row_sums<3>(p, from, to, lane);
+            if (lane == 0) sum += open;
+            if (done) a.y[r + lane] = sum;
+            open = 0.f;
+            r += nd;
+            if (nd < 32) {
+                if ((started_m >> nd) & 1u) open = __shfl_sync(0xffffffffu, sum, nd);
+                break;
+            }
+            s = s2;
+            s_next = s2_next;
+        }
+        __syncwarp();   // p is free for the next tile
+    }
+    for (int i = r + lane; i < r1; i += 32) a.y[i] = 0.f;   // empty rows after the last entry
+}
+
+// The giant rows that begin in ranges [first, first + 32): their pieces in
+// range order (lane-strided, then a fixed tree).
+__device__ __forceinline__ void finish_giants(const NaArgs& a, int first, int lane) {
+    const int k = first + lane;
+    const int mine = k < a.ranges ? __float_as_int(__ldcg(a.carry + kNaSlots * k + 2)) : -1;
+    unsigned todo = __ballot_sync(0xffffffffu, mine >= 0);
+    while (todo) {
+        const int src = __ffs(int(todo)) - 1;
+        todo &= todo - 1;
+        const int row = __shfl_sync(0xffffffffu, mine, src);
+        const int from = first + src;
+        const int end = min(max(__ldg(a.row_ptr + row + 1), 1), a.nnz);
+        const int to = min((end - 1) / a.T, a.ranges - 1);
+        float t = 0.f;
+        for (int j = from + 1 + lane; j <= to; j += 32) t += __ldcg(a.carry + kNaSlots * j);
+        t = warp_total(t);
+        if (lane == 0) a.y[row] = __ldcg(a.carry + kNaSlots * from + 1) + t;
+    }
+}
+
+template <bool kVec, bool kCluster>
+__global__ void __launch_bounds__(kNaWarps * 32, 6) noalloc_spmv_kernel(const NaArgs a) {
+    __shared__ __align__(16) float products[kNaWarps][kNaTile];
+    grid_dep_launch();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = blockIdx.x * kNaWarps + warp;
+    if (k < a.ranges) range_product<kVec>(a, k, lane, products[warp]);
+    if constexpr (kCluster) {
+        // the whole product is this cluster: its pieces are visible after the barrier
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (32 * k < a.ranges) finish_giants(a, 32 * k, lane);
+    }
+}
+
+__global__ void __launch_bounds__(256) noalloc_giants_kernel(const NaArgs a) {
+    grid_dep_wait();
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (32 * warp < a.ranges) finish_giants(a, 32 * warp, threadIdx.x & 31);
+}
+
+template <bool kVec>
+void launch(const NaArgs& a, cudaStream_t stream) {
+    const int blocks = (a.ranges + kNaWarps - 1) / kNaWarps;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(blocks));
+    cfg.blockDim = dim3(kNaWarps * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (blocks <= kNaClusterBlocks) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = unsigned(blocks);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        PB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, noalloc_spmv_kernel<kVec, true>, a));
+        return;
+    }
+    noalloc_spmv_kernel<kVec, false><<<blocks, kNaWarps * 32, 0, stream>>>(a);
+    PB_CUDA_CHECK(cudaGetLastError());
+    // launched while the product drains; it waits for it before it reads the pieces
+    cfg.gridDim = dim3(unsigned((a.ranges + 255) / 256));
+    cfg.blockDim = dim3(256);
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    PB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, noalloc_giants_kernel, a));
 }
 
 // Device address of the scratch array for `dev` (and its SM count), looked up
@@ -220,10 +425,9 @@ void spmv_noalloc(const int32_t* d_row_ptr, const int32_t* d_col_idx, const floa
                   int32_t m, int32_t n, int32_t nnz, const float* d_x, float* d_y,
                   cudaStream_t stream) {
     if (m < 0 || n < 0 || nnz < 0) throw InvalidArgument("negative dimension");
-    if (nnz > (long long)kNoAllocMaxTiles * kNaTile)
+    if (nnz > kNoAllocMaxNnz)
         throw InvalidArgument("pramaan_spmv_noalloc: nnz " + std::to_string(nnz) +
-                              " exceeds the scratch limit of " +
-                              std::to_string((long long)kNoAllocMaxTiles * kNaTile) + " entries");
+                              " exceeds the scratch limit of " + std::to_string(kNoAllocMaxNnz) + " entries");
     if (m == 0) return;
     if (!d_row_ptr || !d_y) throw InvalidArgument("row_ptr and y must not be NULL");
     if (nnz > 0 && (!d_col_idx || !d_values || !d_x || n == 0))
@@ -236,16 +440,18 @@ void spmv_noalloc(const int32_t* d_row_ptr, const int32_t* d_col_idx, const floa
         PB_CUDA_CHECK(cudaMemsetAsync(d_y, 0, size_t(m) * sizeof(float), stream));
         return;
     }
-    const int nt = (nnz + kNaTile - 1) / kNaTile;
-    const int grid = nt < 8 * sms ? nt : 8 * sms;
-    noalloc_spmv_kernel<<<grid, kNaBlock, 0, stream>>>(d_row_ptr, d_col_idx, d_values, m, n, nnz,
-                                                       d_x, d_y, carry);
-    PB_CUDA_CHECK(cudaGetLastError());
-    if (nt > 1) {
-        const int fgrid = (nt + 255) / 256;
-        noalloc_fixup_kernel<<<fgrid, 256, 0, stream>>>(d_row_ptr, m, nnz, carry, d_y);
-        PB_CUDA_CHECK(cudaGetLastError());
-    }
+    // Tiles per range: one, so that a small product spreads over the chip
+    // (1.07 M entries: 16.5 us with one, 25.9 with four), up to four from 4 Mi
+    // entries on, where the ranges fill it anyway and fewer searches pay (4 M
+    // entries: 27.8 us with one, 25.7 with four), more only where the scratch
+    // would not hold the ranges.
+    const int by_size = std::min(std::max(nnz >> 20, 1), 4);
+    const int by_scratch = int((nnz + (long long)kNaTile * kNaMaxRanges - 1) / ((long long)kNaTile * kNaMaxRanges));
+    const int T = kNaTile * std::max(by_size, by_scratch);
+    const NaArgs a{d_row_ptr, d_col_idx, d_values, d_x, d_y, carry, m, n, nnz, T, (nnz + T - 1) / T};
+    const bool vec = ((reinterpret_cast<uintptr_t>(d_col_idx) | reinterpret_cast<uintptr_t>(d_values)) & 15) == 0;
+    if (vec) launch<true>(a, stream);
+    else launch<false>(a, stream);
 }
 
 }  // namespace pb
