@@ -58,6 +58,8 @@ int grid_for(long long work) {
     long long g = (work + kT - 1) / kT;
     return int(std::max<long long>(1, std::min<long long>(g, 148LL * 32)));
 }
+// Grid of the kernels with 8 lanes per row (they stride by the grid).
+int row_grid(long long rows) { return grid_for(rows * 8); }
 #define GNN_STRIDE(i, n) \
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (n); i += (long long)gridDim.x * blockDim.x)
 
@@ -75,9 +77,15 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
     return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
 
-// Stores 32 consecutive FP32 values as BF16 (64 bytes).
-__device__ __forceinline__ void store_bf16x32(bf16* dst, const float (&v)[32]) {
-    uint4* d = reinterpret_cast<uint4*>(dst);
+// Each lane holds its own row of 32 FP32 values; row-wise stores would touch
+// 32 half-used sectors an instruction, so a warp's rows go through 4 KB of
+// shared memory (the tile's consumed TMA stage) and leave as whole 128-byte
+// lines.  Chunk c of 16 bytes of row r lies at chunk c ^ (r & 7): neither side
+// has bank conflicts.
+__device__ __forceinline__ uint4* staged_chunk(uint8_t* buf, int r, int c) {
+    return reinterpret_cast<uint4*>(buf + r * 128 + ((c ^ (r & 7)) << 4));
+}
+__device__ __forceinline__ void stage_bf16x32(uint8_t* buf, int lane, int half, const float (&v)[32]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         uint32_t w[4];
@@ -86,8 +94,25 @@ __device__ __forceinline__ void store_bf16x32(bf16* dst, const float (&v)[32]) {
             __nv_bfloat162 p = __floats2bfloat162_rn(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
             w[e] = *reinterpret_cast<uint32_t*>(&p);
         }
-        d[q] = make_uint4(w[0], w[1], w[2], w[3]);
+        *staged_chunk(buf, lane, half * 4 + q) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+}
+__device__ __forceinline__ void stage_f32x32(uint8_t* buf, int lane, const float (&v)[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(staged_chunk(buf, lane, q)) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+// The staged rows (row0 .. row0 + 31, those below `rows`) to dst + row * pitch bytes, 128 bytes each.
+__device__ __forceinline__ void unstage_rows(uint8_t* buf, int lane, uint8_t* dst, size_t pitch, int row0, int rows) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3), c = lane & 7;
+        const uint4 v = *staged_chunk(buf, r, c);
+        if (row0 + r < rows) *reinterpret_cast<uint4*>(dst + size_t(row0 + r) * pitch + 16 * c) = v;
+    }
+    __syncwarp();
 }
 __device__ __forceinline__ void store_f32x32(float* dst, const float (&v)[32]) {
     float4* d = reinterpret_cast<float4*>(dst);
@@ -101,13 +126,22 @@ __device__ __forceinline__ void drain(uint64_t* bar, bool pending, uint32_t pari
     if (pending) mbar_wait_bounded(bar, parity);
 }
 
+// A node head read off the last layer's rows: hat[r] = base[r] + (w . h[r] + b)
+// (wb: 64 rounded weights, then the bias); wb null: none.
+struct Head {
+    const float* wb = nullptr;
+    const float* base = nullptr;
+    float* hat = nullptr;
+};
+
 // Forward: out[r][0:64] = bf16(relu(X[r] . W^T + b)), X = [rows][128] BF16.
-// Shared memory: X stages 2 x 32 KB, W 16 KB, bias, barriers.
+// Shared memory: X stages 2 x 32 KB, W 16 KB, bias, head weights, barriers.
 struct FwdSmem {
     static constexpr uint32_t kA = 0;
     static constexpr uint32_t kB = 2 * 2 * kBoxBytes;             // 65536
     static constexpr uint32_t kBias = kB + 2 * 64 * 128;          // 81920
-    static constexpr uint32_t kBars = kBias + 64 * 4;
+    static constexpr uint32_t kHead = kBias + 64 * 4;             // 65 floats
+    static constexpr uint32_t kBars = kHead + 68 * 4;
     static constexpr uint32_t kBytes = kBars + 64 + 1024;         // + alignment slack
 };
 constexpr uint32_t kIdescFwd = umma::idesc_bf16<128, 64, false, false>();
@@ -117,7 +151,7 @@ constexpr uint32_t kIdescDw = umma::idesc_bf16<128, 64, true, true>();
 __global__ void __launch_bounds__(kDenseThreads) dense_fwd_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                   const __grid_constant__ CUtensorMap map_w,
                                                                   const float* __restrict__ bias, bf16* __restrict__ out,
-                                                                  int ld_out, int rows, int* status) {
+                                                                  int ld_out, const Head head, int rows, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
     uint8_t* sA = sm + FwdSmem::kA;
@@ -140,7 +174,9 @@ __global__ void __launch_bounds__(kDenseThreads) dense_fwd_kernel(const __grid_c
         umma::tma_prefetch_map(&map_w);
     }
     if (warp == 0) umma::tmem_alloc(tslot, 64);
+    float* shead = reinterpret_cast<float*>(sm + FwdSmem::kHead);
     if (tid < 64) sbias[tid] = bias[tid];
+    if (head.wb && tid < 65) shead[tid] = head.wb[tid];
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -198,14 +234,34 @@ __global__ void __launch_bounds__(kDenseThreads) dense_fwd_kernel(const __grid_c
         __syncwarp();
         const int row = tile * kRowsPerTile + tid;
         const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16);
+        uint8_t* buf = sA + s * 2 * kBoxBytes + warp * 4096;   // the MMAs have read this stage
+        float dot[16];   // the head's dot product, feature pairs folded as a 32-lane xor tree folds them
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float v[32];
             umma::tmem_ld32(taddr + h * 32, v);
 #pragma unroll
             for (int c = 0; c < 32; ++c) v[c] = fmaxf(v[c] + sbias[h * 32 + c], 0.0f);
-            if (row < rows) store_bf16x32(out + size_t(row) * ld_out + h * 32, v);
+            stage_bf16x32(buf, tid & 31, h, v);
+            if (head.wb) {
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    const float2 w = *reinterpret_cast<const float2*>(shead + h * 32 + 2 * q);
+                    const float d = fmaf(w.y, bfr(v[2 * q + 1]), __fmul_rn(w.x, bfr(v[2 * q])));
+                    dot[q] = h == 0 ? d : dot[q] + d;
+                }
+            }
         }
+        if (head.wb && row < rows) {
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int q = 0; q < o; ++q) dot[q] += dot[q + o];
+            head.hat[row] = head.base[row] + (dot[0] + shead[64]);
+        }
+        unstage_rows(buf, tid & 31, reinterpret_cast<uint8_t*>(out), size_t(ld_out) * 2, tile * kRowsPerTile + warp * 32,
+                     rows);
+        fence_proxy_async_smem();   // before the next TMA load into the stage
         umma::fence_before_sync();
         __syncthreads();
     }
@@ -310,17 +366,17 @@ __global__ void __launch_bounds__(kDenseThreads) dense_dx_kernel(const __grid_co
         if (!__syncthreads_and(ok)) { ok = false; break; }
         umma::fence_after_sync();
         __syncwarp();
-        const int row = tile * kRowsPerTile + tid;
         const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16);
+        uint8_t* buf = sA + s * kBoxBytes + warp * 4096;   // the MMAs have read this stage
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             float v[32];
             umma::tmem_ld32(taddr + h * 32, v);
-            if (row < rows) {
-                float* dst = h < 2 ? dh_prev + size_t(row) * 64 + h * 32 : dagg + size_t(row) * 64 + (h - 2) * 32;
-                store_f32x32(dst, v);
-            }
+            stage_f32x32(buf, tid & 31, v);
+            float* dst = h < 2 ? dh_prev + h * 32 : dagg + (h - 2) * 32;
+            unstage_rows(buf, tid & 31, reinterpret_cast<uint8_t*>(dst), 64 * 4, tile * kRowsPerTile + warp * 32, rows);
         }
+        fence_proxy_async_smem();   // before the next TMA load into the stage
         umma::fence_before_sync();
         __syncthreads();
     }
@@ -444,246 +500,541 @@ __global__ void __launch_bounds__(kDenseThreads) dense_dw_kernel(const __grid_co
     }
 }
 
-// dW[g][f] = sum_b partial[b][f][g], blocks in order.
-__global__ void dw_reduce_kernel(const float* __restrict__ partial, int blocks, float* __restrict__ dw) {
-    GNN_STRIDE(t, 64 * 128) {
-        const int g = int(t / 128), f = int(t % 128);
-        float acc = 0.0f;
-        for (int b = 0; b < blocks; ++b) acc += partial[(size_t(b) * 128 + f) * 64 + g];
-        dw[t] = acc;
+// dW[g][f] = sum_b partial[b][f][g].  A block sums 32 consecutive elements,
+// its 8 warps an eighth of the partials each (in order), then the eighths in
+// order: bound by reading the partials (9.7 MB for 296 blocks) out of L2
+// (one thread per element over all partials took 43 us on 16 windows).
+__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, int blocks,
+                                                        float* __restrict__ dw) {
+    __shared__ float sums[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.x * 32 + lane;   // f * 64 + g
+    float acc = 0.0f;
+#pragma unroll 8
+    for (int b = warp; b < blocks; b += 8) acc += __ldcg(partial + size_t(b) * (128 * 64) + t);
+    sums[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) acc += sums[w][lane];
+        dw[(t & 63) * 128 + (t >> 6)] = acc;
     }
 }
 
 // ---------------------------------------------------------------------------
 // CUDA-core kernels
 // ---------------------------------------------------------------------------
-// h0[r][o] = bf16(relu(sum_f W[o][f] feat[r][f] + b[o]))
 constexpr int kF = kGnnFeat;
-__global__ void input_layer_kernel(const float* __restrict__ feat, int nodes, const float* __restrict__ w,
-                                   bf16* __restrict__ out, int ld) {
-    __shared__ float sw[64 * kF + 64];
-    for (int t = threadIdx.x; t < 64 * kF + 64; t += blockDim.x) sw[t] = w[t];
-    __syncthreads();
-    GNN_STRIDE(t, (long long)nodes * 64) {
-        const long long r = t >> 6;
-        const int o = int(t & 63);
-        const float* f = feat + r * kF;
-        float acc = 0.0f;
+
+// One warp-wide load of 8 BF16 features per lane: 8 lanes hold a row of 64.
+__device__ __forceinline__ uint4 ld_row8(const bf16* h, size_t row, int ld, int sub) {
+    return *reinterpret_cast<const uint4*>(h + row * ld + 8 * sub);
+}
+__device__ __forceinline__ void unpack8(uint4 v, float (&f)[8]) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int q = 0; q < kF; ++q) acc = fmaf(sw[o * kF + q], f[q], acc);
-        acc += sw[64 * kF + o];
-        out[r * ld + o] = __float2bfloat16_rn(fmaxf(acc, 0.0f));
+    for (int q = 0; q < 4; ++q) {
+        f[2 * q] = __uint_as_float(w[q] << 16);
+        f[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+    }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
+        w[q] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// h0[r][o] = bf16(relu(sum_f W[o][f] feat[r][f] + b[o])).  A lane keeps the
+// weights of two outputs in registers and walks 32 nodes whose features its
+// warp staged in shared memory: bound by instruction issue (28 per node and
+// warp; a thread per output with the weights in shared memory took 70).
+__global__ void __launch_bounds__(256) input_layer_kernel(const float* __restrict__ feat, int nodes,
+                                                          const float* __restrict__ w, bf16* __restrict__ out, int ld) {
+    constexpr int kPad = 12;   // floats per staged node: three 16-byte reads
+    __shared__ __align__(16) float stage[8][32 * kPad];
+    const int lane = threadIdx.x & 31;
+    float* s = stage[threadIdx.x >> 5];
+    float w0[kF], w1[kF];
+#pragma unroll
+    for (int q = 0; q < kF; ++q) {
+        w0[q] = w[2 * lane * kF + q];
+        w1[q] = w[(2 * lane + 1) * kF + q];
+    }
+    const float b0 = w[64 * kF + 2 * lane], b1 = w[64 * kF + 2 * lane + 1];
+    const int warps = gridDim.x * 8;
+    for (int base = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; base < nodes; base += warps * 32) {
+        const int cnt = min(32, nodes - base);
+        for (int t = lane; t < cnt * kF; t += 32) s[t / kF * kPad + t % kF] = feat[size_t(base) * kF + t];
+        __syncwarp();
+#pragma unroll 4
+        for (int i = 0; i < cnt; ++i) {
+            const float4* f4 = reinterpret_cast<const float4*>(s + i * kPad);
+            const float4 fa = f4[0], fb = f4[1];
+            const float f[kF] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w, s[i * kPad + 8]};
+            float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll
+            for (int q = 0; q < kF; ++q) {
+                a0 = fmaf(w0[q], f[q], a0);
+                a1 = fmaf(w1[q], f[q], a1);
+            }
+            *reinterpret_cast<__nv_bfloat162*>(out + size_t(base + i) * ld + 2 * lane) =
+                __floats2bfloat162_rn(fmaxf(a0 + b0, 0.0f), fmaxf(a1 + b1, 0.0f));
+        }
+        __syncwarp();
     }
 }
 
-// out[r][64:128] = bf16(sum_{e in row r} coef[e] h[col[e]][0:64]); one warp per row.
-__global__ void aggregate_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                 const float* __restrict__ coef, const bf16* __restrict__ h, int ldh,
-                                 bf16* __restrict__ out, int ldo, int rows) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
+// out[r][64:128] = bf16(sum_{e in row r} coef[e] h[col[e]][0:64]), entries in
+// order.  8 lanes per row, 8 features each, so a warp works on four rows and
+// an entry is one 16-byte load per lane; kEdges entries are in flight before
+// the first is added.  Bound by those gathers' round trips: rows hold two to
+// six entries.
+template <int kEdges>
+__global__ void __launch_bounds__(256) aggregate_kernel(const int* __restrict__ rp, const int* __restrict__ col,
+                                                        const float* __restrict__ coef, const bf16* __restrict__ h,
+                                                        int ldh, bf16* __restrict__ out, int ldo, int rows) {
+    const int sub = threadIdx.x & 7;
+    for (int r = (blockIdx.x * 256 + threadIdx.x) >> 3; r < rows; r += gridDim.x * 32) {
         const int beg = rp[r], end = rp[r + 1];
-        float a0 = 0.0f, a1 = 0.0f;
-        for (int base = beg; base < end; base += 32) {
-            const int e = base + lane;
-            const int c = e < end ? col[e] : 0;
-            const float w = e < end ? coef[e] : 0.0f;
-            const int cnt = min(32, end - base);
-            for (int t = 0; t < cnt; ++t) {
-                const int cc = __shfl_sync(0xffffffffu, c, t);
-                const float ww = __shfl_sync(0xffffffffu, w, t);
-                const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(h + size_t(cc) * ldh + 2 * lane);
-                a0 = fmaf(ww, __low2float(v), a0);
-                a1 = fmaf(ww, __high2float(v), a1);
+        float a[8] = {};
+        for (int e = beg; e < end; e += kEdges) {
+            int c[kEdges];
+            float w[kEdges];
+            uint4 v[kEdges];
+#pragma unroll
+            for (int u = 0; u < kEdges; ++u) {
+                c[u] = e + u < end ? col[e + u] : 0;
+                w[u] = e + u < end ? coef[e + u] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < kEdges; ++u) v[u] = e + u < end ? ld_row8(h, size_t(c[u]), ldh, sub) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < kEdges; ++u) {
+                if (e + u < end) {
+                    float f[8];
+                    unpack8(v[u], f);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) a[q] = fmaf(w[u], f[q], a[q]);
+                }
             }
         }
-        *reinterpret_cast<__nv_bfloat162*>(out + size_t(r) * ldo + 64 + 2 * lane) = __floats2bfloat162_rn(a0, a1);
+        *reinterpret_cast<uint4*>(out + size_t(r) * ldo + 64 + 8 * sub) = pack8(a);
     }
 }
 
-// dh[r][0:64] += sum_{e in row r} coef[e] dagg[col[e]][0:64] (FP32).
-__global__ void aggregate_bwd_kernel(const int* __restrict__ rp, const int* __restrict__ col,
-                                     const float* __restrict__ coef, const float* __restrict__ dagg,
-                                     float* __restrict__ dh, int rows) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
-        const int beg = rp[r], end = rp[r + 1];
-        float a0 = 0.0f, a1 = 0.0f;
-        for (int base = beg; base < end; base += 32) {
-            const int e = base + lane;
-            const int c = e < end ? col[e] : 0;
-            const float w = e < end ? coef[e] : 0.0f;
-            const int cnt = min(32, end - base);
-            for (int t = 0; t < cnt; ++t) {
-                const int cc = __shfl_sync(0xffffffffu, c, t);
-                const float ww = __shfl_sync(0xffffffffu, w, t);
-                const float2 v = *reinterpret_cast<const float2*>(dagg + size_t(cc) * 64 + 2 * lane);
-                a0 = fmaf(ww, v.x, a0);
-                a1 = fmaf(ww, v.y, a1);
-            }
-        }
-        float2* d = reinterpret_cast<float2*>(dh + size_t(r) * 64 + 2 * lane);
-        float2 o = *d;
-        o.x += a0;
-        o.y += a1;
-        *d = o;
-    }
-}
-
-// out[r] = base[r] + (w . h[r] + b) (w: 64 rounded weights, then the bias); one warp per node.
-__global__ void head_kernel(const bf16* __restrict__ h, int nodes, const float* __restrict__ wb,
-                            const float* __restrict__ base, float* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < nodes; r += warps) {
-        const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(h + size_t(r) * 64 + 2 * lane);
-        float p = fmaf(wb[2 * lane + 1], __high2float(v), wb[2 * lane] * __low2float(v));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-        if (lane == 0) out[r] = base[r] + (p + wb[64]);
-    }
-}
-
-// Sums over the nodes of each chunk: part[c][t] = sum_{r in chunk c} F(r, t).
-template <class F>
-__global__ void chunk_kernel(F f, int width, const int* __restrict__ begin, int chunks, float* __restrict__ part) {
-    for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
-        const int b = begin[c], e = begin[c + 1];
-        for (int t = threadIdx.x; t < width; t += blockDim.x) {
-            float acc = 0.0f;
-            for (int r = b; r < e; ++r) acc += f(r, t);
-            part[size_t(c) * width + t] = acc;
-        }
-    }
-}
-
-struct PoolF {          // h [r][64] BF16
-    const bf16* h;
-    __device__ float operator()(int r, int t) const { return bf(h[size_t(r) * 64 + t]); }
+// One side's nodes cut into chunks of one LP each.
+struct Chunks {
+    const int* begin;      // [chunks + 1]
+    const int* lp_first;   // [K + 1]
+    int chunks;
 };
-struct SqErrF {         // (hat - target)^2 / count of the node's LP
+
+// part[c][t] = sum of feature t of h over the nodes of chunk c, in node order:
+// the variable side's chunks, then the constraint side's.  A warp per chunk, a
+// lane two features, kPoolAhead rows in flight (one dependent add per row is
+// the definition's order, so only the loads overlap).
+constexpr int kPoolAhead = 32;
+__global__ void __launch_bounds__(128) pool_kernel(const bf16* __restrict__ hv, Chunks cv, const bf16* __restrict__ hc,
+                                                   Chunks cc, float* __restrict__ part) {
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < cv.chunks + cc.chunks; c += warps) {
+        const bool v = c < cv.chunks;
+        const int* begin = v ? cv.begin + c : cc.begin + (c - cv.chunks);
+        const bf16* h = v ? hv : hc;
+        const int b = begin[0], e = begin[1];
+        float a0 = 0.0f, a1 = 0.0f;
+        auto row = [&](int r) { return __ldg(reinterpret_cast<const uint32_t*>(h + size_t(r) * 64 + 2 * lane)); };
+        auto add = [&](uint32_t x) {
+            a0 += __uint_as_float(x << 16);
+            a1 += __uint_as_float(x & 0xffff0000u);
+        };
+        int r = b;
+        for (; r + kPoolAhead <= e; r += kPoolAhead) {
+            uint32_t x[kPoolAhead];
+#pragma unroll
+            for (int u = 0; u < kPoolAhead; ++u) x[u] = row(r + u);
+#pragma unroll
+            for (int u = 0; u < kPoolAhead; ++u) add(x[u]);
+        }
+#pragma unroll 4
+        for (; r < e; ++r) add(row(r));
+        *reinterpret_cast<float2*>(part + size_t(c) * 64 + 2 * lane) = make_float2(a0, a1);
+    }
+}
+
+// Sum of src[c * stride] for c in [b, e), in order, 32 loads in flight.
+__device__ __forceinline__ float ordered_sum(const float* __restrict__ src, int b, int e, int stride) {
+    float acc = 0.0f;
+    int c = b;
+    for (; c + 32 <= e; c += 32) {
+        float v[32];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) v[u] = src[size_t(c + u) * stride];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) acc += v[u];
+    }
+#pragma unroll 8
+    for (; c < e; ++c) acc += src[size_t(c) * stride];
+    return acc;
+}
+
+// Per LP (a block): pooled means of both sides from the chunk sums, chunks in
+// order, and rho_k = w_w . pooled_k + b_w (128 weights, then the bias).
+__global__ void __launch_bounds__(128) pooled_rho_kernel(const float* __restrict__ part, Chunks cv, Chunks cc,
+                                                         const float* __restrict__ inv_n,
+                                                         const float* __restrict__ inv_m,
+                                                         const float* __restrict__ wb, int K,
+                                                         float* __restrict__ pooled, float* __restrict__ rho) {
+    __shared__ float mean[128];
+    const int t = threadIdx.x, lane = t & 31;
+    for (int k = blockIdx.x; k < K; k += gridDim.x) {
+        const bool v = t < 64;
+        const int* first = v ? cv.lp_first + k : cc.lp_first + k;
+        const float* src = part + (v ? size_t(t) : size_t(cv.chunks) * 64 + size_t(t - 64));
+        const float p = ordered_sum(src, first[0], first[1], 64) * (v ? inv_n[k] : inv_m[k]);
+        mean[t] = p;
+        pooled[size_t(k) * 128 + t] = p;
+        __syncthreads();
+        if (t < 32) {
+            float d = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) d = fmaf(wb[4 * lane + q], mean[4 * lane + q], d);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if (lane == 0) rho[k] = d + wb[128];
+        }
+        __syncthreads();
+    }
+}
+
+// One side of a loss or head gradient: predictions, targets, the LP of every
+// node and the LP's loss weight.
+struct HeadSide {
     const float* hat;
     const float* tgt;
     const int* lp;
-    const float* inv;
-    __device__ float operator()(int r, int) const {
-        const float d = hat[r] - tgt[r];
-        return d * d * inv[lp[r]];
-    }
+    const float* lw;
 };
-struct HeadGradF {      // t < 64: d[r] h[r][t]; t == 64: d[r]
-    const bf16* h;
-    const float* d;
-    __device__ float operator()(int r, int t) const { return t < 64 ? d[r] * bf(h[size_t(r) * 64 + t]) : d[r]; }
-};
-struct BiasGradF {      // dz [r][64] BF16
-    const bf16* dz;
-    __device__ float operator()(int r, int t) const { return bf(dz[size_t(r) * 64 + t]); }
-};
-constexpr int kInW = 64 * kF;   // input-layer weights; the 64 biases follow
-constexpr int kWide = kInW + 64; // widest chunk partial
 
-// Input-layer gradient partials: part[c][o*9 + q] = sum_{r in chunk c} dz0[r][o] f[r][q],
-// part[c][kInW + o] = sum_r dz0[r][o], with dz0 = dh0 masked by h0 > 0.  One
-// thread per output feature o (coalesced dh / h0 reads), nodes in order.
-__global__ void inlayer_grad_kernel(const float* __restrict__ dh, const bf16* __restrict__ h0, int ldh0,
-                                    const float* __restrict__ feat, const int* __restrict__ begin, int chunks,
-                                    float* __restrict__ part) {
-    const int o = threadIdx.x;   // blockDim.x == 64
-    for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
-        float acc[kF + 1];
-#pragma unroll
-        for (int q = 0; q <= kF; ++q) acc[q] = 0.0f;
-        for (int r = begin[c]; r < begin[c + 1]; ++r) {
-            const float g = bf(h0[size_t(r) * ldh0 + o]) > 0.0f ? dh[size_t(r) * 64 + o] : 0.0f;
-            const float* f = feat + size_t(r) * kF;
-#pragma unroll
-            for (int q = 0; q < kF; ++q) acc[q] += g * f[q];
-            acc[kF] += g;
-        }
-        float* dst = part + size_t(c) * kWide;
-#pragma unroll
-        for (int q = 0; q < kF; ++q) dst[o * kF + q] = acc[q];
-        dst[kInW + o] = acc[kF];
-    }
-}
-
-// out[k][t] = scale_k * sum_{c in LP k's chunks} part[c][t]
-__global__ void lp_sum_kernel(const float* __restrict__ part, int width, const int* __restrict__ lp_first, int K,
-                              const float* __restrict__ inv, float* __restrict__ out, int ld_out) {
-    GNN_STRIDE(t, (long long)K * width) {
-        const int k = int(t / width), w = int(t % width);
-        float acc = 0.0f;
-        for (int c = lp_first[k]; c < lp_first[k + 1]; ++c) acc += part[size_t(c) * width + w];
-        out[size_t(k) * ld_out + w] = inv ? acc * inv[k] : acc;
-    }
-}
-
-// Ordered group sums: dst[g][t] = sum_{r in [64g, 64g+64)} src[r][t].
-__global__ void group_sum_kernel(const float* __restrict__ src, int rows, int width, float* __restrict__ dst) {
-    const int groups = (rows + 63) / 64;
-    GNN_STRIDE(t, (long long)groups * width) {
-        const int g = int(t / width), w = int(t % width);
-        float acc = 0.0f;
-        const int e = min(rows, 64 * g + 64);
-        for (int r = 64 * g; r < e; ++r) acc += src[size_t(r) * width + w];
-        dst[t] = acc;
-    }
-}
-
-// rho_k = w_w . pooled_k + b_w (128 weights, then the bias); one warp per LP.
-__global__ void rho_kernel(const float* __restrict__ pooled, int K, const float* __restrict__ wb,
-                           float* __restrict__ rho) {
+// part[c] = sum over the nodes of chunk c of (hat - target)^2 lw, in node
+// order (variable side, then constraint side): a warp loads 32 terms at a
+// time and every lane adds them in order.
+__global__ void __launch_bounds__(128) square_error_kernel(HeadSide sv, Chunks cv, HeadSide sc, Chunks cc,
+                                                           float* __restrict__ part) {
     const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long k = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; k < K; k += warps) {
-        float p = 0.0f;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < cv.chunks + cc.chunks; c += warps) {
+        const bool v = c < cv.chunks;
+        const int* begin = v ? cv.begin + c : cc.begin + (c - cv.chunks);
+        const HeadSide s = v ? sv : sc;
+        const int b = begin[0], e = begin[1];
+        static_assert(kGnnChunk % 32 == 0, "chunks are whole warps but for an LP's last");
+        float sq[kGnnChunk / 32], lw[kGnnChunk / 32];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) p = fmaf(wb[4 * lane + q], pooled[size_t(k) * 128 + 4 * lane + q], p);
+        for (int u = 0; u < kGnnChunk / 32; ++u) {
+            const int r = b + u * 32 + lane;
+            const float d = r < e ? s.hat[r] - s.tgt[r] : 0.0f;
+            sq[u] = __fmul_rn(d, d);
+            lw[u] = r < e ? s.lw[s.lp[r]] : 0.0f;
+        }
+        float acc = 0.0f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-        if (lane == 0) rho[k] = p + wb[128];
+        for (int u = 0; u < kGnnChunk / 32; ++u) {
+            const int cnt = min(32, e - b - u * 32);
+            for (int t = 0; t < cnt; ++t)
+                acc = fmaf(__shfl_sync(0xffffffffu, sq[u], t), __shfl_sync(0xffffffffu, lw[u], t), acc);
+        }
+        if (lane == 0) part[c] = acc;
     }
 }
 
-// d[r] = 2 (hat[r] - tgt[r]) inv[lp[r]] / K
-__global__ void head_delta_kernel(const float* __restrict__ hat, const float* __restrict__ tgt,
-                                  const int* __restrict__ lp, const float* __restrict__ inv, float inv_k, int nodes,
-                                  float* __restrict__ d) {
-    GNN_STRIDE(r, nodes) d[r] = 2.0f * (hat[r] - tgt[r]) * inv[lp[r]] * inv_k;
-}
-
-// dh[r][f] = d[r] w[f] + drho[lp] ww[f] inv[lp]
-__global__ void head_back_kernel(const float* __restrict__ d, const int* __restrict__ lp, const float* __restrict__ w,
-                                 const float* __restrict__ drho, const float* __restrict__ ww,
-                                 const float* __restrict__ inv, int nodes, float* __restrict__ dh) {
-    GNN_STRIDE(t, (long long)nodes * 64) {
-        const long long r = t >> 6;
-        const int f = int(t & 63);
-        const int k = lp[r];
-        dh[t] = fmaf(d[r], w[f], drho[k] * ww[f] * inv[k]);
+// One block: each LP's x and y terms from the chunk sums (chunks in order),
+// the loss (LPs in order, FP64) and drho_k = 2 (rho_k - tw_k) / K; with
+// `grad` the gradient of the primal-weight head, sum_k drho_k [pooled_k ; 1].
+__global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ part, Chunks cv, Chunks cc,
+                                                   const float* __restrict__ rho, const float* __restrict__ tw, int K,
+                                                   float inv_k, const float* __restrict__ pooled,
+                                                   float* __restrict__ sums, float* __restrict__ drho,
+                                                   float* __restrict__ grad, double* __restrict__ loss) {
+    for (int t = threadIdx.x; t < 2 * K; t += blockDim.x) {
+        const bool v = t < K;
+        const int* first = v ? cv.lp_first + t : cc.lp_first + (t - K);
+        sums[t] = ordered_sum(part + (v ? 0 : cv.chunks), first[0], first[1], 1);
     }
-}
-
-// out[t] = sum_k drho[k] pooled[k][t] (t < 128), sum_k drho[k] (t = 128); LPs in order.
-__global__ void rho_grad_kernel(const float* __restrict__ pooled, const float* __restrict__ drho, int K,
-                                float* __restrict__ out) {
+    for (int k = threadIdx.x; k < K; k += blockDim.x)
+        drho[k] = __fmul_rn(float(2.0 * (double(rho[k]) - double(tw[k]))), inv_k);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double total = 0.0;
+        for (int k = 0; k < K; ++k) {
+            const double dw = double(rho[k]) - double(tw[k]);
+            total = __dadd_rn(total, __dadd_rn(__dadd_rn(double(sums[k]), double(sums[K + k])), __dmul_rn(dw, dw)));
+        }
+        *loss = total / K;
+    }
+    if (!grad) return;
     for (int t = threadIdx.x; t < 129; t += blockDim.x) {
         float acc = 0.0f;
         for (int k = 0; k < K; ++k) acc += t < 128 ? drho[k] * pooled[size_t(k) * 128 + t] : drho[k];
-        out[t] = acc;
+        grad[t] = acc;
     }
 }
 
-// dz[r][f] = bf16(h[r][f] > 0 ? dh[r][f] : 0)
-__global__ void dz_kernel(const float* __restrict__ dh, const bf16* __restrict__ h, int ldh, int nodes,
-                          bf16* __restrict__ dz) {
-    GNN_STRIDE(t, (long long)nodes * 64) {
-        const long long r = t >> 6;
-        const int f = int(t & 63);
-        dz[t] = __float2bfloat16_rn(bf(h[r * ldh + f]) > 0.0f ? dh[t] : 0.0f);
+// ---- gradient partials ------------------------------------------------------
+// Every block of the node kernels below writes one row of gpart_; the columns:
+constexpr int kColBias = 0;                              // dense layers' biases, (2 l + side) * 64
+constexpr int kColHead = kColBias + 2 * kGnnLayers * 64; // w_x, b_x, then w_y, b_y
+constexpr int kColIn = kColHead + 2 * 65;                // W_vin, b_vin, then W_cin, b_cin
+constexpr int kInWide = 64 * kF + 64;
+constexpr int kGradCols = kColIn + 2 * kInWide;
+
+// Adds each thread's N partial vectors of 8 features (features 8 (tid & 7) ...)
+// over the block into row[n * stride + feature], groups in a fixed order.
+template <int N>
+__device__ __forceinline__ void block_feature_sums(float (&acc)[N][8], float* __restrict__ row, const int (&at)[N]) {
+    __shared__ float sums[8][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            acc[n][q] += __shfl_xor_sync(0xffffffffu, acc[n][q], 8);
+            acc[n][q] += __shfl_xor_sync(0xffffffffu, acc[n][q], 16);
+        }
+        __syncthreads();
+        if (lane < 8) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) sums[warp][8 * lane + q] = acc[n][q];
+        }
+        __syncthreads();
+        if (threadIdx.x < 64) {
+            float t = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) t += sums[w][threadIdx.x];
+            row[at[n] + threadIdx.x] = t;
+        }
+    }
+}
+
+struct NodeBackward {
+    int rows;
+    // dh_r += sum_{e in row r} coef[e] dagg[col[e]]; rp null: no such terms
+    const int* rp;
+    const int* col;
+    const float* coef;
+    const float* dagg;
+    float* dh;               // kHead: not read; kFinal: written
+    const bf16* h;           // the layer's output rows
+    int ldh;
+    bf16* dz;                // !kFinal: bf16(h > 0 ? dh : 0)
+    float* part;             // gpart_
+    int col_bias, col_head;  // columns of the bias and head gradients
+    // kHead: dh from the node head and the pooled primal-weight head
+    HeadSide side;
+    float inv_k;
+    const float* w;          // head weights [64]
+    const float* ww;         // this side's half of the primal-weight head [64]
+    const float* drho;
+    const float* inv;        // 1 / nodes of the LP
+};
+
+// One pass over a side's nodes on the way back: the gradient dh of every
+// hidden row (the dense layer's own part, or the heads' with kHead, plus the
+// other side's aggregation terms, entries in order), masked by the ReLU into
+// the BF16 dz the dense gradients read, with the bias and head gradients
+// summed on the way.  dh never returns to memory except for the input layer
+// (kFinal).  8 lanes per row, 8 features each; bound by the FP32 rows it reads
+// (256 bytes per node and per entry).
+constexpr int kBackEdges = 4;
+template <bool kHead, bool kFinal>
+__global__ void __launch_bounds__(256) node_backward_kernel(const NodeBackward a) {
+    const int sub = threadIdx.x & 7;
+    float sums[kHead ? 2 : 1][8] = {};   // bias; head weights
+    float dsum = 0.0f;
+    float w[8], ww[8];
+    if constexpr (kHead) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            w[q] = a.w[8 * sub + q];
+            ww[q] = a.ww[8 * sub + q];
+        }
+    }
+    for (int r = (blockIdx.x * 256 + threadIdx.x) >> 3; r < a.rows; r += gridDim.x * 32) {
+        const int beg = a.rp ? a.rp[r] : 0, end = a.rp ? a.rp[r + 1] : 0;
+        float dh[8], h[8];
+        uint4 hv = make_uint4(0, 0, 0, 0);
+        if constexpr (!kFinal) hv = ld_row8(a.h, size_t(r), a.ldh, sub);
+        float d = 0.0f;
+        if constexpr (kHead) {
+            const int k = a.side.lp[r];
+            d = 2.0f * (a.side.hat[r] - a.side.tgt[r]) * a.side.lw[k] * a.inv_k;
+            const float dr = a.drho[k], iv = a.inv[k];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) dh[q] = fmaf(d, w[q], dr * ww[q] * iv);
+        } else {
+            const float4* p = reinterpret_cast<const float4*>(a.dh + size_t(r) * 64 + 8 * sub);
+            const float4 x = p[0], y = p[1];
+            dh[0] = x.x; dh[1] = x.y; dh[2] = x.z; dh[3] = x.w;
+            dh[4] = y.x; dh[5] = y.y; dh[6] = y.z; dh[7] = y.w;
+        }
+        float g[8] = {};
+        for (int e = beg; e < end; e += kBackEdges) {
+            int c[kBackEdges];
+            float f[kBackEdges];
+            float4 x[kBackEdges], y[kBackEdges];
+#pragma unroll
+            for (int u = 0; u < kBackEdges; ++u) {
+                c[u] = e + u < end ? a.col[e + u] : 0;
+                f[u] = e + u < end ? a.coef[e + u] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < kBackEdges; ++u) {
+                const float4* p = reinterpret_cast<const float4*>(a.dagg + size_t(c[u]) * 64 + 8 * sub);
+                x[u] = e + u < end ? p[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                y[u] = e + u < end ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < kBackEdges; ++u) {
+                if (e + u < end) {
+                    g[0] = fmaf(f[u], x[u].x, g[0]); g[1] = fmaf(f[u], x[u].y, g[1]);
+                    g[2] = fmaf(f[u], x[u].z, g[2]); g[3] = fmaf(f[u], x[u].w, g[3]);
+                    g[4] = fmaf(f[u], y[u].x, g[4]); g[5] = fmaf(f[u], y[u].y, g[5]);
+                    g[6] = fmaf(f[u], y[u].z, g[6]); g[7] = fmaf(f[u], y[u].w, g[7]);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) dh[q] += g[q];
+        if constexpr (kFinal) {
+            float4* p = reinterpret_cast<float4*>(a.dh + size_t(r) * 64 + 8 * sub);
+            p[0] = make_float4(dh[0], dh[1], dh[2], dh[3]);
+            p[1] = make_float4(dh[4], dh[5], dh[6], dh[7]);
+        } else {
+            unpack8(hv, h);
+            float z[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) z[q] = h[q] > 0.0f ? dh[q] : 0.0f;
+            const uint4 packed = pack8(z);
+            *reinterpret_cast<uint4*>(a.dz + size_t(r) * 64 + 8 * sub) = packed;
+            unpack8(packed, z);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) sums[0][q] += z[q];
+            if constexpr (kHead) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) sums[1][q] = fmaf(d, h[q], sums[1][q]);
+                dsum += d;   // the same value in the 8 lanes of a row
+            }
+        }
+    }
+    if constexpr (!kFinal) {
+        float* row = a.part + size_t(blockIdx.x) * kGradCols;
+        if constexpr (kHead) {
+            const int at[2] = {a.col_bias, a.col_head};
+            block_feature_sums<2>(sums, row, at);
+            __shared__ float ds[8];
+            dsum += __shfl_xor_sync(0xffffffffu, dsum, 8);
+            dsum += __shfl_xor_sync(0xffffffffu, dsum, 16);
+            if ((threadIdx.x & 31) == 0) ds[threadIdx.x >> 5] = dsum;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                float t = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) t += ds[q];
+                row[a.col_head + 64] = t;
+            }
+        } else {
+            const int at[1] = {a.col_bias};
+            block_feature_sums<1>(sums, row, at);
+        }
+    }
+}
+
+// Input-layer gradient: row[o*9 + q] = sum_r dz0[r][o] f[r][q], row[576 + o] =
+// sum_r dz0[r][o] over the block's nodes, dz0 = dh masked by h0 > 0 (FP32).
+// Four threads share an output feature o and take every fourth node; bound by
+// the rows read (420 bytes per node).
+constexpr int kInTile = 64;   // nodes whose features are staged at a time
+__global__ void __launch_bounds__(256) inlayer_grad_kernel(const float* __restrict__ dh, const bf16* __restrict__ h0,
+                                                           int ldh0, const float* __restrict__ feat, int nodes,
+                                                           float* __restrict__ part, int col) {
+    __shared__ float f[kInTile * kF];
+    __shared__ float sums[4][64];
+    const int o = threadIdx.x & 63, g = threadIdx.x >> 6;
+    float acc[kF + 1] = {};
+    for (int base = blockIdx.x * kInTile; base < nodes; base += gridDim.x * kInTile) {
+        const int cnt = min(kInTile, nodes - base);
+        __syncthreads();
+        for (int t = threadIdx.x; t < cnt * kF; t += 256) f[t] = feat[size_t(base) * kF + t];
+        float z[kInTile / 4];
+#pragma unroll
+        for (int u = 0; u < kInTile / 4; ++u) {
+            const int i = min(4 * u + g, cnt - 1);   // past the end: the last node, not added
+            const size_t r = size_t(base + i);
+            const float hv = bf(h0[r * ldh0 + o]), d = dh[r * 64 + o];
+            z[u] = hv > 0.0f ? d : 0.0f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kInTile / 4; ++u) {
+            const int i = 4 * u + g;
+            if (i < cnt) {
+#pragma unroll
+                for (int q = 0; q < kF; ++q) acc[q] = fmaf(z[u], f[i * kF + q], acc[q]);
+                acc[kF] += z[u];
+            }
+        }
+    }
+    float* row = part + size_t(blockIdx.x) * kGradCols + col;
+#pragma unroll
+    for (int q = 0; q <= kF; ++q) {
+        __syncthreads();
+        sums[g][o] = acc[q];
+        __syncthreads();
+        if (g == 0) row[q < kF ? o * kF + q : 64 * kF + o] = ((sums[0][o] + sums[1][o]) + sums[2][o]) + sums[3][o];
+    }
+}
+
+// Place of gradient column c in the parameter vector; -1: a constraint-side
+// column of a graph without constraints.
+__device__ __forceinline__ int grad_place(int c, bool has_c) {
+    if (c < kColHead) {
+        const int d = c / 64;
+        return (d & 1) == 0 && !has_c ? -1 : GnnParams::layer_b(d >> 1, d & 1) + c % 64;
+    }
+    if (c < kColIn) {
+        const int t = c - kColHead;
+        return t < 65 ? GnnParams::kHeadX + t : has_c ? GnnParams::kHeadY + (t - 65) : -1;
+    }
+    const int t = c - kColIn;
+    return t < kInWide ? GnnParams::kVinW + t : has_c ? GnnParams::kCinW + (t - kInWide) : -1;
+}
+static_assert(GnnParams::kVinB == GnnParams::kVinW + 64 * kF && GnnParams::kCinB == GnnParams::kCinW + 64 * kF,
+              "an input layer's bias follows its weights");
+
+// The blocks' rows of gpart_ added per column: 8 warps an eighth of the rows
+// each, then the eighths, in order.
+__global__ void __launch_bounds__(256) grad_total_kernel(const float* __restrict__ part, int rows, bool has_c,
+                                                         float* __restrict__ grad) {
+    __shared__ float sums[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
+    const int place = c < kGradCols ? grad_place(c, has_c) : -1;
+    float acc = 0.0f;
+    if (place >= 0) {
+#pragma unroll 8
+        for (int b = warp; b < rows; b += 8) acc += __ldcg(part + size_t(b) * kGradCols + c);
+    }
+    sums[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && place >= 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) acc += sums[w][lane];
+        grad[place] = acc;
     }
 }
 
@@ -725,6 +1076,9 @@ float uniform(uint64_t& s, float a) {
     const double u = double(splitmix(s) >> 11) * (1.0 / 9007199254740992.0);
     return float((2.0 * u - 1.0) * a);
 }
+
+// Blocks of the node kernels that leave one row of gradient partials each.
+int grad_blocks(int dev) { return 4 * device_sm_count(dev); }
 
 int dense_blocks(int dev, int rows, int per_sm) {
     const int tiles = (rows + kRowsPerTile - 1) / kRowsPerTile;
@@ -1054,7 +1408,7 @@ void GnnModel::copy_grad(float* host) const {
 
 void GnnModel::ensure_workspace(const GnnGraph& g) {
     const size_t m = size_t(std::max(g.m, 1)), n = size_t(std::max(g.n, 1)), k = size_t(std::max(g.K, 1));
-    const size_t chunks = size_t(std::max(std::max(g.cchunks, g.rchunks), 1));
+    const size_t chunks = size_t(std::max(g.cchunks + g.rchunks, 1));
     if (m > cap_m_) {
         for (auto& b : xc_) b.alloc(m * 128);
         hc3_.alloc(m * 64);
@@ -1076,38 +1430,20 @@ void GnnModel::ensure_workspace(const GnnGraph& g) {
     }
     if (k > cap_k_) {
         pooled_.alloc(k * 128);
-        rho_.alloc(k * 4);         // rho, drho, loss_w, spare
-        lp_sums_.alloc(k * 4);
+        rho_.alloc(k * 2);         // rho, drho
+        lp_sums_.alloc(k * 2);
         cap_k_ = k;
     }
     if (chunks > cap_chunks_) {
-        // chunk partials and two ping-pong halves, up to kWide columns wide
-        part_.alloc(chunks * kWide * 2 + kWide);
+        part_.alloc(chunks * 64);
         cap_chunks_ = chunks;
     }
-    if (wpart_.size() == 0) wpart_.alloc(size_t(2 * device_sm_count(dev_)) * 128 * 64);
-}
-
-namespace {
-// Deterministic total over `rows` partial rows of `width` columns; the result
-// lands in `out` (device).  `scratch` holds at least rows/64 + 1 rows.
-void ordered_total(const float* part, int rows, int width, float* scratch, float* out, cudaStream_t st) {
-    const float* cur = part;
-    float* bufs[2] = {scratch, scratch + size_t((rows + 63) / 64 + 1) * width};
-    int b = 0;
-    while (rows > 1) {
-        const int groups = (rows + 63) / 64;
-        float* dst = groups == 1 ? out : bufs[b];
-        group_sum_kernel<<<grid_for((long long)groups * width), kT, 0, st>>>(cur, rows, width, dst);
-        PB_CUDA_CHECK(cudaGetLastError());
-        cur = dst;
-        rows = groups;
-        b ^= 1;
+    if (wpart_.size() == 0) {
+        wpart_.alloc(size_t(2 * device_sm_count(dev_)) * 128 * 64);
+        gpart_.alloc(size_t(grad_blocks(dev_)) * kGradCols);
+        loss_.alloc(1);
     }
-    if (rows == 1 && cur != out)
-        PB_CUDA_CHECK(cudaMemcpyAsync(out, cur, size_t(width) * 4, cudaMemcpyDeviceToDevice, st));
 }
-}  // namespace
 
 void GnnModel::forward(const GnnGraph& g) {
     last_ = &g;
@@ -1116,27 +1452,31 @@ void GnnModel::forward(const GnnGraph& g) {
     PB_CUDA_CHECK(cudaMemsetAsync(status_.get(), 0, 4, st_));
     const float* pr = pr_.get();
     // input layers
-    input_layer_kernel<<<grid_for((long long)g.n * 64), kT, 0, st_>>>(g.fv.get(), g.n, pr + GnnParams::kVinW,
-                                                                      xv_[0].get(), 128);
+    input_layer_kernel<<<grid_for(g.n), kT, 0, st_>>>(g.fv.get(), g.n, pr + GnnParams::kVinW, xv_[0].get(), 128);
     if (g.m > 0)
-        input_layer_kernel<<<grid_for((long long)g.m * 64), kT, 0, st_>>>(g.fc.get(), g.m, pr + GnnParams::kCinW,
-                                                                          xc_[0].get(), 128);
+        input_layer_kernel<<<grid_for(g.m), kT, 0, st_>>>(g.fc.get(), g.m, pr + GnnParams::kCinW, xc_[0].get(), 128);
     PB_CUDA_CHECK(cudaGetLastError());
     for (int l = 0; l < kGnnLayers; ++l) {
         bf16* out_c = l + 1 < kGnnLayers ? xc_[l + 1].get() : hc3_.get();
         bf16* out_v = l + 1 < kGnnLayers ? xv_[l + 1].get() : hv3_.get();
         const int ldo = l + 1 < kGnnLayers ? 128 : 64;
+        Head head_c, head_v;
+        if (l + 1 == kGnnLayers) {
+            head_c = {pr + GnnParams::kHeadY, g.base_y.get(), yhat_.get()};
+            head_v = {pr + GnnParams::kHeadX, g.base_x.get(), xhat_.get()};
+        }
         if (g.m > 0) {
-            aggregate_kernel<<<grid_for((long long)g.m * 32), kT, 0, st_>>>(g.rp.get(), g.ci.get(), g.coef_r.get(),
-                                                                            xv_[l].get(), 128, xc_[l].get(), 128, g.m);
+            // constraint rows hold five entries or more, columns two or three
+            aggregate_kernel<8><<<row_grid(g.m), kT, 0, st_>>>(g.rp.get(), g.ci.get(), g.coef_r.get(), xv_[l].get(),
+                                                               128, xc_[l].get(), 128, g.m);
             PB_CUDA_CHECK(cudaGetLastError());
             const CUtensorMap mx = make_bf16_tile_map(xc_[l].get(), g.m, 128, 128, 128);
             const CUtensorMap mw = make_bf16_tile_map(w_.get() + size_t(2 * l) * 64 * 128, 64, 128, 128, 64);
             dense_fwd_kernel<<<dense_blocks(dev_, g.m, 2), kDenseThreads, FwdSmem::kBytes, st_>>>(
-                mx, mw, pr + GnnParams::layer_b(l, 0), out_c, ldo, g.m, status_.get());
+                mx, mw, pr + GnnParams::layer_b(l, 0), out_c, ldo, head_c, g.m, status_.get());
             PB_CUDA_CHECK(cudaGetLastError());
-            aggregate_kernel<<<grid_for((long long)g.n * 32), kT, 0, st_>>>(g.tp.get(), g.ti.get(), g.tcoef_c.get(),
-                                                                            out_c, ldo, xv_[l].get(), 128, g.n);
+            aggregate_kernel<4><<<row_grid(g.n), kT, 0, st_>>>(g.tp.get(), g.ti.get(), g.tcoef_c.get(), out_c, ldo,
+                                                               xv_[l].get(), 128, g.n);
         } else {
             // no constraints: the aggregated half of the variable input is zero
             PB_CUDA_CHECK(cudaMemset2DAsync(xv_[l].get() + 64, 256, 0, 128, size_t(g.n), st_));
@@ -1145,32 +1485,16 @@ void GnnModel::forward(const GnnGraph& g) {
         const CUtensorMap mx = make_bf16_tile_map(xv_[l].get(), g.n, 128, 128, 128);
         const CUtensorMap mw = make_bf16_tile_map(w_.get() + size_t(2 * l + 1) * 64 * 128, 64, 128, 128, 64);
         dense_fwd_kernel<<<dense_blocks(dev_, g.n, 2), kDenseThreads, FwdSmem::kBytes, st_>>>(
-            mx, mw, pr + GnnParams::layer_b(l, 1), out_v, ldo, g.n, status_.get());
+            mx, mw, pr + GnnParams::layer_b(l, 1), out_v, ldo, head_v, g.n, status_.get());
         PB_CUDA_CHECK(cudaGetLastError());
     }
-    // heads
-    head_kernel<<<grid_for((long long)g.n * 32), kT, 0, st_>>>(hv3_.get(), g.n, pr + GnnParams::kHeadX,
-                                                               g.base_x.get(), xhat_.get());
-    if (g.m > 0)
-        head_kernel<<<grid_for((long long)g.m * 32), kT, 0, st_>>>(hc3_.get(), g.m, pr + GnnParams::kHeadY,
-                                                                   g.base_y.get(), yhat_.get());
-    PB_CUDA_CHECK(cudaGetLastError());
     // pooled means per LP, then rho
-    float* part = part_.get();
-    chunk_kernel<<<std::min(g.cchunks, 148 * 8), 64, 0, st_>>>(PoolF{hv3_.get()}, 64, g.cchunk_begin.get(), g.cchunks,
-                                                              part);
-    lp_sum_kernel<<<grid_for((long long)g.K * 64), kT, 0, st_>>>(part, 64, g.clp_first.get(), g.K, g.inv_n.get(),
-                                                                pooled_.get(), 128);
-    PB_CUDA_CHECK(cudaGetLastError());
-    if (g.m > 0) {
-        chunk_kernel<<<std::min(g.rchunks, 148 * 8), 64, 0, st_>>>(PoolF{hc3_.get()}, 64, g.rchunk_begin.get(),
-                                                                  g.rchunks, part);
-        lp_sum_kernel<<<grid_for((long long)g.K * 64), kT, 0, st_>>>(part, 64, g.rlp_first.get(), g.K, g.inv_m.get(),
-                                                                    pooled_.get() + 64, 128);
-    } else {
-        PB_CUDA_CHECK(cudaMemset2DAsync(pooled_.get() + 64, 512, 0, 256, size_t(g.K), st_));
-    }
-    rho_kernel<<<grid_for((long long)g.K * 32), kT, 0, st_>>>(pooled_.get(), g.K, pr + GnnParams::kHeadW, rho_.get());
+    const Chunks cv{g.cchunk_begin.get(), g.clp_first.get(), g.cchunks};
+    const Chunks cc{g.rchunk_begin.get(), g.rlp_first.get(), g.rchunks};
+    pool_kernel<<<std::min((cv.chunks + cc.chunks + 3) / 4, 148 * 16), 128, 0, st_>>>(hv3_.get(), cv, hc3_.get(), cc,
+                                                                                  part_.get());
+    pooled_rho_kernel<<<std::min(g.K, 148 * 8), 128, 0, st_>>>(part_.get(), cv, cc, g.inv_n.get(), g.inv_m.get(),
+                                                             pr + GnnParams::kHeadW, g.K, pooled_.get(), rho_.get());
     PB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -1179,132 +1503,91 @@ double GnnModel::backward(const GnnGraph& g, bool grad) {
     if (!g.has_targets) throw InvalidArgument("gnn: the graph has no targets");
     if (g.K == 0) return 0.0;
     const float* pr = pr_.get();
-    float* part = part_.get();
-    float* scratch = part_.get() + cap_chunks_ * kWide;
     float* G = g_.get();
     const float inv_k = 1.0f / float(g.K);
     float* drho = rho_.get() + cap_k_;
+    const Chunks cv{g.cchunk_begin.get(), g.clp_first.get(), g.cchunks};
+    const Chunks cc{g.rchunk_begin.get(), g.rlp_first.get(), g.rchunks};
+    const HeadSide sv{xhat_.get(), g.tx.get(), g.lp_col.get(), g.lw_x.get()};
+    const HeadSide sc{yhat_.get(), g.ty.get(), g.lp_row.get(), g.lw_y.get()};
     // ---- loss per LP: x and y terms from chunk sums, omega term from rho ----
-    std::vector<float> hl(size_t(3) * g.K);
-    chunk_kernel<<<std::min(g.cchunks, 148 * 8), 32, 0, st_>>>(SqErrF{xhat_.get(), g.tx.get(), g.lp_col.get(),
-                                                                      g.lw_x.get()},
-                                                              1, g.cchunk_begin.get(), g.cchunks, part);
-    lp_sum_kernel<<<grid_for(g.K), kT, 0, st_>>>(part, 1, g.clp_first.get(), g.K, nullptr, lp_sums_.get(), 1);
-    if (g.m > 0) {
-        chunk_kernel<<<std::min(g.rchunks, 148 * 8), 32, 0, st_>>>(
-            SqErrF{yhat_.get(), g.ty.get(), g.lp_row.get(), g.lw_y.get()}, 1, g.rchunk_begin.get(), g.rchunks, part);
-        lp_sum_kernel<<<grid_for(g.K), kT, 0, st_>>>(part, 1, g.rlp_first.get(), g.K, nullptr,
-                                                    lp_sums_.get() + cap_k_, 1);
-    } else {
-        PB_CUDA_CHECK(cudaMemsetAsync(lp_sums_.get() + cap_k_, 0, size_t(g.K) * 4, st_));
-    }
+    if (grad) PB_CUDA_CHECK(cudaMemsetAsync(G, 0, g_.bytes(), st_));
+    square_error_kernel<<<std::min((cv.chunks + cc.chunks + 3) / 4, 148 * 16), 128, 0, st_>>>(sv, cv, sc, cc,
+                                                                                          part_.get());
+    loss_kernel<<<1, 256, 0, st_>>>(part_.get(), cv, cc, rho_.get(), g.tw.get(), g.K, inv_k, pooled_.get(),
+                                    lp_sums_.get(), drho, grad ? G + GnnParams::kHeadW : nullptr, loss_.get());
     PB_CUDA_CHECK(cudaGetLastError());
-    std::vector<float> hrho(size_t(g.K)), htw(size_t(g.K));
-    PB_CUDA_CHECK(cudaMemcpyAsync(hl.data(), lp_sums_.get(), size_t(g.K) * 4, cudaMemcpyDeviceToHost, st_));
-    PB_CUDA_CHECK(cudaMemcpyAsync(hl.data() + g.K, lp_sums_.get() + cap_k_, size_t(g.K) * 4, cudaMemcpyDeviceToHost, st_));
-    PB_CUDA_CHECK(cudaMemcpyAsync(hrho.data(), rho_.get(), size_t(g.K) * 4, cudaMemcpyDeviceToHost, st_));
-    PB_CUDA_CHECK(cudaMemcpyAsync(htw.data(), g.tw.get(), size_t(g.K) * 4, cudaMemcpyDeviceToHost, st_));
-    int hstatus = 0;
-    PB_CUDA_CHECK(cudaMemcpyAsync(&hstatus, status_.get(), 4, cudaMemcpyDeviceToHost, st_));
-    PB_CUDA_CHECK(cudaStreamSynchronize(st_));
-    if (hstatus & kDevErrTimeout) throw DeviceTimeout("gnn: a tensor-core tile wait exceeded its time limit");
+    if (grad) {
+        const int blocks = grad_blocks(dev_);
+        // Variable-side rows of the layer that `dh` belongs to; `head`: the last layer, from the heads.
+        auto base = [&](bool head, bool v, int layer) {
+            NodeBackward a{};
+            a.rows = v ? g.n : g.m;
+            a.dh = v ? dhv_.get() : dhc_.get();
+            a.dagg = dagg_.get();
+            a.ldh = layer + 1 < kGnnLayers ? 128 : 64;
+            a.h = layer + 1 < kGnnLayers ? (v ? xv_[layer + 1].get() : xc_[layer + 1].get())
+                                         : (v ? hv3_.get() : hc3_.get());
+            a.dz = dz_.get();
+            a.part = gpart_.get();
+            a.col_bias = kColBias + (2 * layer + (v ? 1 : 0)) * 64;
+            if (head) {
+                a.col_head = kColHead + (v ? 0 : 65);
+                a.side = v ? sv : sc;
+                a.inv_k = inv_k;
+                a.w = pr + (v ? GnnParams::kHeadX : GnnParams::kHeadY);
+                a.ww = pr + GnnParams::kHeadW + (v ? 0 : 64);
+                a.drho = drho;
+                a.inv = v ? g.inv_n.get() : g.inv_m.get();
+            }
+            return a;
+        };
+        auto dense_back = [&](int layer, bool v, const bf16* x, float* dh) {
+            const int rows = v ? g.n : g.m, side = v ? 1 : 0;
+            const int wblocks = dense_blocks(dev_, rows, 2);
+            const CUtensorMap mx = make_bf16_tile_map(x, rows, 128, 128, 128);
+            const CUtensorMap mz = make_bf16_tile_map(dz_.get(), rows, 64, 64, 128);
+            const CUtensorMap mwt = make_bf16_tile_map(wt_.get() + size_t(2 * layer + side) * 64 * 128, 128, 64, 64, 128);
+            dense_dw_kernel<<<wblocks, kDenseThreads, DwSmem::kBytes, st_>>>(mx, mz, wpart_.get(), rows, status_.get());
+            PB_CUDA_CHECK(cudaGetLastError());
+            dw_reduce_kernel<<<64 * 128 / 32, 256, 0, st_>>>(wpart_.get(), wblocks, G + GnnParams::layer_w(layer, side));
+            dense_dx_kernel<<<dense_blocks(dev_, rows, 4), kDenseThreads, DxSmem::kBytes, st_>>>(
+                mz, mwt, dh, dagg_.get(), rows, status_.get());
+            PB_CUDA_CHECK(cudaGetLastError());
+        };
+        // ---- message-passing layers, last to first ----
+        node_backward_kernel<true, false><<<blocks, 256, 0, st_>>>(base(true, true, kGnnLayers - 1));
+        PB_CUDA_CHECK(cudaGetLastError());
+        for (int l = kGnnLayers - 1; l >= 0; --l) {
+            dense_back(l, true, xv_[l].get(), dhv_.get());
+            NodeBackward v = base(false, true, l - 1);
+            if (g.m > 0) {
+                // agg_v backward: dh_c[i] += sum_j A_ij/(s_a deg_j) dagg_v[j]
+                const bool head = l + 1 == kGnnLayers;
+                NodeBackward c = base(head, false, l);
+                c.rp = g.rp.get(); c.col = g.ci.get(); c.coef = g.coef_c.get();
+                if (head) node_backward_kernel<true, false><<<blocks, 256, 0, st_>>>(c);
+                else node_backward_kernel<false, false><<<blocks, 256, 0, st_>>>(c);
+                PB_CUDA_CHECK(cudaGetLastError());
+                dense_back(l, false, xc_[l].get(), dhc_.get());
+                // agg_c backward: dh_v[j] += sum_i A_ij/(s_a deg_i) dagg_c[i]
+                v.rp = g.tp.get(); v.col = g.ti.get(); v.coef = g.tcoef_r.get();
+            }
+            if (l > 0) node_backward_kernel<false, false><<<blocks, 256, 0, st_>>>(v);
+            else if (g.m > 0) node_backward_kernel<false, true><<<blocks, 256, 0, st_>>>(v);
+            PB_CUDA_CHECK(cudaGetLastError());
+        }
+        // ---- input layers ----
+        inlayer_grad_kernel<<<blocks, 256, 0, st_>>>(dhv_.get(), xv_[0].get(), 128, g.fv.get(), g.n, gpart_.get(), kColIn);
+        if (g.m > 0)
+            inlayer_grad_kernel<<<blocks, 256, 0, st_>>>(dhc_.get(), xc_[0].get(), 128, g.fc.get(), g.m, gpart_.get(),
+                                                         kColIn + kInWide);
+        grad_total_kernel<<<(kGradCols + 31) / 32, 256, 0, st_>>>(gpart_.get(), blocks, g.m > 0, G);
+        PB_CUDA_CHECK(cudaGetLastError());
+    }
     double loss = 0.0;
-    std::vector<float> hdrho(size_t(g.K));
-    for (int k = 0; k < g.K; ++k) {
-        const double dw = double(hrho[size_t(k)]) - double(htw[size_t(k)]);
-        loss += double(hl[size_t(k)]) + double(hl[size_t(g.K + k)]) + dw * dw;
-        hdrho[size_t(k)] = float(2.0 * dw) * inv_k;
-    }
-    loss /= g.K;
-    if (!grad) return loss;
-
-    // ---- heads ----
-    PB_CUDA_CHECK(cudaMemsetAsync(G, 0, g_.bytes(), st_));
-    PB_CUDA_CHECK(cudaMemcpyAsync(drho, hdrho.data(), size_t(g.K) * 4, cudaMemcpyHostToDevice, st_));
-    float* dxh = dagg_.get();                     // per-node head deltas (scratch)
-    float* dyh = dagg_.get() + cap_n_;
-    head_delta_kernel<<<grid_for(g.n), kT, 0, st_>>>(xhat_.get(), g.tx.get(), g.lp_col.get(), g.lw_x.get(), inv_k,
-                                                    g.n, dxh);
-    chunk_kernel<<<std::min(g.cchunks, 148 * 8), 96, 0, st_>>>(HeadGradF{hv3_.get(), dxh}, 65, g.cchunk_begin.get(),
-                                                              g.cchunks, part);
-    ordered_total(part, g.cchunks, 65, scratch, G + GnnParams::kHeadX, st_);
-    if (g.m > 0) {
-        head_delta_kernel<<<grid_for(g.m), kT, 0, st_>>>(yhat_.get(), g.ty.get(), g.lp_row.get(), g.lw_y.get(),
-                                                        inv_k, g.m, dyh);
-        chunk_kernel<<<std::min(g.rchunks, 148 * 8), 96, 0, st_>>>(HeadGradF{hc3_.get(), dyh}, 65,
-                                                                  g.rchunk_begin.get(), g.rchunks, part);
-        ordered_total(part, g.rchunks, 65, scratch, G + GnnParams::kHeadY, st_);
-    }
-    // w_w, b_w: sum_k drho_k [pooled_k ; 1]
-    rho_grad_kernel<<<1, 160, 0, st_>>>(pooled_.get(), drho, g.K, G + GnnParams::kHeadW);
-    PB_CUDA_CHECK(cudaGetLastError());
-    head_back_kernel<<<grid_for((long long)g.n * 64), kT, 0, st_>>>(dxh, g.lp_col.get(), pr + GnnParams::kHeadX, drho,
-                                                                   pr + GnnParams::kHeadW, g.inv_n.get(), g.n,
-                                                                   dhv_.get());
-    if (g.m > 0)
-        head_back_kernel<<<grid_for((long long)g.m * 64), kT, 0, st_>>>(dyh, g.lp_row.get(), pr + GnnParams::kHeadY,
-                                                                       drho, pr + GnnParams::kHeadW + 64,
-                                                                       g.inv_m.get(), g.m, dhc_.get());
-    PB_CUDA_CHECK(cudaGetLastError());
-
-    // ---- message-passing layers, last to first ----
-    const int wblocks_v = dense_blocks(dev_, g.n, 2), wblocks_c = dense_blocks(dev_, std::max(g.m, 1), 2);
-    for (int l = kGnnLayers - 1; l >= 0; --l) {
-        const bf16* out_c = l + 1 < kGnnLayers ? xc_[l + 1].get() : hc3_.get();
-        const bf16* out_v = l + 1 < kGnnLayers ? xv_[l + 1].get() : hv3_.get();
-        const int ldo = l + 1 < kGnnLayers ? 128 : 64;
-        // variable side
-        dz_kernel<<<grid_for((long long)g.n * 64), kT, 0, st_>>>(dhv_.get(), out_v, ldo, g.n, dz_.get());
-        chunk_kernel<<<std::min(g.cchunks, 148 * 8), 64, 0, st_>>>(BiasGradF{dz_.get()}, 64, g.cchunk_begin.get(),
-                                                                  g.cchunks, part);
-        ordered_total(part, g.cchunks, 64, scratch, G + GnnParams::layer_b(l, 1), st_);
-        {
-            const CUtensorMap mx = make_bf16_tile_map(xv_[l].get(), g.n, 128, 128, 128);
-            const CUtensorMap mz = make_bf16_tile_map(dz_.get(), g.n, 64, 64, 128);
-            dense_dw_kernel<<<wblocks_v, kDenseThreads, DwSmem::kBytes, st_>>>(mx, mz, wpart_.get(), g.n, status_.get());
-            PB_CUDA_CHECK(cudaGetLastError());
-            dw_reduce_kernel<<<grid_for(64 * 128), kT, 0, st_>>>(wpart_.get(), wblocks_v, G + GnnParams::layer_w(l, 1));
-            const CUtensorMap mwt = make_bf16_tile_map(wt_.get() + size_t(2 * l + 1) * 64 * 128, 128, 64, 64, 128);
-            dense_dx_kernel<<<dense_blocks(dev_, g.n, 4), kDenseThreads, DxSmem::kBytes, st_>>>(
-                mz, mwt, dhv_.get(), dagg_.get(), g.n, status_.get());
-            PB_CUDA_CHECK(cudaGetLastError());
-        }
-        if (g.m > 0) {
-            // agg_v backward: dh_c[i] += sum_j A_ij/(s_a deg_j) dagg_v[j]
-            aggregate_bwd_kernel<<<grid_for((long long)g.m * 32), kT, 0, st_>>>(g.rp.get(), g.ci.get(),
-                                                                                g.coef_c.get(), dagg_.get(),
-                                                                                dhc_.get(), g.m);
-            // constraint side
-            dz_kernel<<<grid_for((long long)g.m * 64), kT, 0, st_>>>(dhc_.get(), out_c, ldo, g.m, dz_.get());
-            chunk_kernel<<<std::min(g.rchunks, 148 * 8), 64, 0, st_>>>(BiasGradF{dz_.get()}, 64,
-                                                                      g.rchunk_begin.get(), g.rchunks, part);
-            ordered_total(part, g.rchunks, 64, scratch, G + GnnParams::layer_b(l, 0), st_);
-            const CUtensorMap mx = make_bf16_tile_map(xc_[l].get(), g.m, 128, 128, 128);
-            const CUtensorMap mz = make_bf16_tile_map(dz_.get(), g.m, 64, 64, 128);
-            dense_dw_kernel<<<wblocks_c, kDenseThreads, DwSmem::kBytes, st_>>>(mx, mz, wpart_.get(), g.m, status_.get());
-            PB_CUDA_CHECK(cudaGetLastError());
-            dw_reduce_kernel<<<grid_for(64 * 128), kT, 0, st_>>>(wpart_.get(), wblocks_c, G + GnnParams::layer_w(l, 0));
-            const CUtensorMap mwt = make_bf16_tile_map(wt_.get() + size_t(2 * l) * 64 * 128, 128, 64, 64, 128);
-            dense_dx_kernel<<<dense_blocks(dev_, g.m, 4), kDenseThreads, DxSmem::kBytes, st_>>>(
-                mz, mwt, dhc_.get(), dagg_.get(), g.m, status_.get());
-            PB_CUDA_CHECK(cudaGetLastError());
-            // agg_c backward: dh_v[j] += sum_i A_ij/(s_a deg_i) dagg_c[i]
-            aggregate_bwd_kernel<<<grid_for((long long)g.n * 32), kT, 0, st_>>>(g.tp.get(), g.ti.get(),
-                                                                                g.tcoef_r.get(), dagg_.get(),
-                                                                                dhv_.get(), g.n);
-            PB_CUDA_CHECK(cudaGetLastError());
-        }
-    }
-    // ---- input layers ----
-    inlayer_grad_kernel<<<std::min(g.cchunks, 148 * 16), 64, 0, st_>>>(dhv_.get(), xv_[0].get(), 128, g.fv.get(),
-                                                                         g.cchunk_begin.get(), g.cchunks, part);
-    ordered_total(part, g.cchunks, kWide, scratch, G + GnnParams::kVinW, st_);
-    if (g.m > 0) {
-        inlayer_grad_kernel<<<std::min(g.rchunks, 148 * 16), 64, 0, st_>>>(dhc_.get(), xc_[0].get(), 128, g.fc.get(),
-                                                                           g.rchunk_begin.get(), g.rchunks, part);
-        ordered_total(part, g.rchunks, kWide, scratch, G + GnnParams::kCinW, st_);
-    }
-    PB_CUDA_CHECK(cudaGetLastError());
+    int hstatus = 0;
+    PB_CUDA_CHECK(cudaMemcpyAsync(&loss, loss_.get(), sizeof(double), cudaMemcpyDeviceToHost, st_));
     PB_CUDA_CHECK(cudaMemcpyAsync(&hstatus, status_.get(), 4, cudaMemcpyDeviceToHost, st_));
     PB_CUDA_CHECK(cudaStreamSynchronize(st_));
     if (hstatus & kDevErrTimeout) throw DeviceTimeout("gnn: a tensor-core tile wait exceeded its time limit");

@@ -48,8 +48,8 @@
 // staged by TMA with the 128-byte swizzle, FP32 accumulators in tensor
 // memory): forward H = relu(X W^T + b), input gradient dX = dZ W and weight
 // gradient dW^T = X^T dZ (MN-major operands, per-CTA partials reduced in a
-// fixed order).  The aggregations are warp-per-node gathers over the CSR of
-// A and of its transpose, so the backward pass is a gather too and every
+// fixed order).  The aggregations are gathers (8 lanes per node) over the CSR
+// of A and of its transpose, so the backward pass is a gather too and every
 // reduction is deterministic.
 #pragma once
 
@@ -162,6 +162,8 @@ private:
     DevBuf<float> dhc_, dhv_, dagg_;                            // [rows][64]
     DevBuf<float> xhat_, yhat_, pooled_, rho_;
     DevBuf<float> part_, lp_sums_, wpart_;
+    DevBuf<float> gpart_;                  // gradient partials, one row per block of the node kernels
+    DevBuf<double> loss_;
     const GnnGraph* last_ = nullptr;
 };
 
