@@ -145,10 +145,13 @@ struct EpiPrimalAdapt {
 // written per element on the iterations that ask for it (fpr != nullptr).
 constexpr float kHalpernReflection = 1.0f;
 
-// Halpern weight of LP q at iteration offset of the interval.
-__device__ __forceinline__ float halpern_weight_lp(const int* iter_base, int offset, const int* restart_iter, int q) {
-    const long long k = (long long)(*iter_base) + offset - restart_iter[q];
+// Halpern weight k iterations after a restart, and that of LP q at iteration
+// offset of the interval.
+__device__ __forceinline__ float halpern_weight_of(long long k) {
     return k <= 0 ? 0.5f : float(double(k + 1) / double(k + 2));
+}
+__device__ __forceinline__ float halpern_weight_lp(const int* iter_base, int offset, const int* restart_iter, int q) {
+    return halpern_weight_of((long long)(*iter_base) + offset - restart_iter[q]);
 }
 __device__ __forceinline__ float halpern_weight(const int* iter_base, int offset, const int* restart_iter,
                                                 const int* lp, int i) {
@@ -192,21 +195,25 @@ struct EpiPrimalHalpern {
         return in;
     }
     __device__ In load(int j) const { return load(j, halpern_weight(iter_base, offset, restart_iter, lp, j)); }
-    __device__ void store(State&, int j, const In& in, float aty) const {
-        if (!(in.t > 0.0f)) {        // a frozen LP keeps its iterate
-            x_bar[j] = in.x_prev;
-            if (fpr) fpr[j] = 0.0;
-            return;
-        }
+    // The new x of a column, its extrapolation in xb, and its residual term in
+    // *f when f is given.
+    __device__ static float update(const In& in, float aty, float& xb, double* f) {
+        const bool live = in.t > 0.0f;   // a frozen LP keeps its iterate
         const float g = __fadd_rn(in.c, aty);
         const float xt = fminf(fmaxf(__fmaf_rn(-in.t, g, in.x_prev), in.lo), in.hi);
-        x_bar[j] = __fmaf_rn(2.0f, xt, -in.x_prev);
+        xb = live ? __fmaf_rn(2.0f, xt, -in.x_prev) : in.x_prev;
         const float refl = __fmaf_rn(1.0f + kHalpernReflection, xt, -kHalpernReflection * in.x_prev);
-        x[j] = __fmaf_rn(in.w, __fsub_rn(refl, in.a), in.a);
-        if (fpr) {
+        if (f) {
             const double d = double(in.x_prev) - double(xt);
-            fpr[j] = d * d / double(in.t);
+            *f = live ? d * d / double(in.t) : 0.0;
         }
+        return live ? __fmaf_rn(in.w, __fsub_rn(refl, in.a), in.a) : in.x_prev;
+    }
+    __device__ void store(State&, int j, const In& in, float aty) const {
+        float xb;
+        const float xn = update(in, aty, xb, fpr ? fpr + j : nullptr);
+        x_bar[j] = xb;
+        x[j] = xn;
     }
     __device__ void apply(State& st, int j, float aty) const { store(st, j, load(j), aty); }
     __device__ void finish(State&, int) const {}
@@ -244,26 +251,25 @@ struct EpiDualHalpern {
         return in;
     }
     __device__ In load(int i) const { return load(i, halpern_weight(iter_base, offset, restart_iter, lp, i)); }
-    __device__ void store(State&, int i, const In& in, float ad) const {
+    // The new e of a row, and its residual term in *f when f is given.
+    __device__ static float update(const In& in, float ad, double* f) {
         const float s = in.s;
         const float e_prev = in.e_prev;
-        float en = e_prev;
-        if (s > 0.0f) {
-            const float ym = in.ym;
-            const float q = __fdiv_rn(__fadd_rn(ym, e_prev), s);
-            const float hi = __fadd_rn(ad, in.hi);
-            const float lo = __fadd_rn(ad, in.lo);
-            if (__fadd_rn(q, hi) > 0.0f) en = __fmaf_rn(s, hi, e_prev);
-            else if (__fadd_rn(q, lo) < 0.0f) en = __fmaf_rn(s, lo, e_prev);
-            else en = -ym;
-        }
+        const float ym = in.ym;
+        const float q = __fdiv_rn(__fadd_rn(ym, e_prev), s);
+        const float hi = __fadd_rn(ad, in.hi);
+        const float lo = __fadd_rn(ad, in.lo);
+        const bool above = __fadd_rn(q, hi) > 0.0f, below = __fadd_rn(q, lo) < 0.0f;
+        const float moved = __fmaf_rn(s, above ? hi : lo, e_prev);
+        const float en = s > 0.0f ? (above || below ? moved : -ym) : e_prev;
         const float refl = __fmaf_rn(1.0f + kHalpernReflection, en, -kHalpernReflection * e_prev);
-        e[i] = __fmaf_rn(in.w, __fsub_rn(refl, in.a), in.a);
-        if (fpr) {
+        if (f) {
             const double d = double(e_prev) - double(en);
-            fpr[i] = s > 0.0f ? d * d / double(s) : 0.0;
+            *f = s > 0.0f ? d * d / double(s) : 0.0;
         }
+        return __fmaf_rn(in.w, __fsub_rn(refl, in.a), in.a);
     }
+    __device__ void store(State&, int i, const In& in, float ad) const { e[i] = update(in, ad, fpr ? fpr + i : nullptr); }
     __device__ void apply(State& st, int i, float ad) const { store(st, i, load(i), ad); }
     __device__ void finish(State&, int) const {}
 };

@@ -30,46 +30,90 @@ enum : int {
 
 // ---- per-LP reductions ---------------------------------------------------
 
-// One block per chunk: sums (or maxima) of `width` <= 4 interleaved values.
-template <bool kMax>
-__global__ void chunk_reduce_kernel(const double* __restrict__ contrib, int width,
-                                    const int* __restrict__ begin, double* __restrict__ out) {
-    __shared__ double sh[4][256];
-    const int c = blockIdx.x;
-    const int b = begin[c], e = begin[c + 1];
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = b + threadIdx.x; i < e; i += blockDim.x)
-        for (int s = 0; s < width; ++s) {
-            const double v = contrib[size_t(i) * width + s];
-            acc[s] = kMax ? fmax(acc[s], v) : acc[s] + v;
-        }
-    for (int s = 0; s < width; ++s) sh[s][threadIdx.x] = acc[s];
+// One array of per-element contributions to be summed (or maximised) per LP.
+struct ReduceJob {
+    const double* contrib;     // `width` <= 4 interleaved values per element
+    const int* begin;          // the side's chunks
+    const int* lp_first;
+    int chunks, width, out_off;
+    int first;                 // the job's first chunk among all jobs'
+};
+constexpr int kReduceJobs = 6;
+struct ReduceJobs {
+    ReduceJob job[kReduceJobs];
+    int n;
+};
+
+// One block per chunk of one array.  A thread adds every 256th element in
+// order, then a halving tree over the threads: 16 elements a thread, whose
+// loads are issued before they are added (a check interval ends in six of
+// these reductions; one launch each with a load per add took 13.6 us each).
+template <bool kMax, int kWidth>
+__device__ __forceinline__ void chunk_reduce(const double* __restrict__ contrib, int b, int e, double* __restrict__ out) {
+    __shared__ double sh[kWidth][256];
+    constexpr int kAhead = kWidth == 1 ? 16 : 4;
+    double acc[kWidth];
+#pragma unroll
+    for (int s = 0; s < kWidth; ++s) acc[s] = 0.0;
+    for (int i = b + int(threadIdx.x); i < e; i += 256 * kAhead) {
+        double v[kAhead][kWidth];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int s = 0; s < kWidth; ++s) v[u][s] = contrib[size_t(min(i + 256 * u, e - 1)) * kWidth + s];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int s = 0; s < kWidth; ++s)
+                if (i + 256 * u < e) acc[s] = kMax ? fmax(acc[s], v[u][s]) : acc[s] + v[u][s];
+    }
+#pragma unroll
+    for (int s = 0; s < kWidth; ++s) sh[s][threadIdx.x] = acc[s];
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int s = 0; s < width; ++s) {
+    for (int w = 128; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+#pragma unroll
+            for (int s = 0; s < kWidth; ++s) {
                 const double a = sh[s][threadIdx.x], o = sh[s][threadIdx.x + w];
                 sh[s][threadIdx.x] = kMax ? fmax(a, o) : a + o;
             }
+        }
         __syncthreads();
     }
-    if (threadIdx.x < width) out[size_t(c) * width + threadIdx.x] = sh[threadIdx.x][0];
+    if (threadIdx.x < kWidth) out[threadIdx.x] = sh[threadIdx.x][0];
 }
 
-// One thread per (LP, slot): the LP's chunks in order.
 template <bool kMax>
-__global__ void lp_reduce_kernel(const double* __restrict__ chunk_out, int width,
-                                 const int* __restrict__ lp_first, int K, double* __restrict__ out,
-                                 int out_off) {
+__global__ void __launch_bounds__(256) chunk_reduce_kernel(const ReduceJobs jobs, double* __restrict__ out) {
+    int q = 0;
+    while (q + 1 < jobs.n && int(blockIdx.x) >= jobs.job[q + 1].first) ++q;
+    const ReduceJob& J = jobs.job[q];
+    const int c = int(blockIdx.x) - J.first;
+    const int b = J.begin[c], e = J.begin[c + 1];
+    double* o = out + size_t(blockIdx.x) * 4;
+    switch (J.width) {
+        case 1: chunk_reduce<kMax, 1>(J.contrib, b, e, o); break;
+        case 2: chunk_reduce<kMax, 2>(J.contrib, b, e, o); break;
+        case 3: chunk_reduce<kMax, 3>(J.contrib, b, e, o); break;
+        default: chunk_reduce<kMax, 4>(J.contrib, b, e, o); break;
+    }
+}
+
+// One thread per (job, LP, slot): the LP's chunks in order.
+template <bool kMax>
+__global__ void lp_reduce_kernel(const ReduceJobs jobs, const double* __restrict__ chunk_out, int K,
+                                 double* __restrict__ out) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= K * width) return;
-    const int k = t / width, s = t % width;
+    const int q = t / (K * 4), k = t / 4 % K, s = t % 4;
+    if (q >= jobs.n) return;
+    const ReduceJob& J = jobs.job[q];
+    if (s >= J.width) return;
     double acc = 0.0;
-    for (int c = lp_first[k]; c < lp_first[k + 1]; ++c) {
-        const double v = chunk_out[size_t(c) * width + s];
+    for (int c = J.lp_first[k]; c < J.lp_first[k + 1]; ++c) {
+        const double v = chunk_out[size_t(J.first + c) * 4 + s];
         acc = kMax ? fmax(acc, v) : acc + v;
     }
-    out[size_t(k) * kOutWidth + out_off + s] = acc;
+    out[size_t(k) * kOutWidth + J.out_off + s] = acc;
 }
 
 // ---- per-element epilogues writing contributions ---------------------------
@@ -492,7 +536,7 @@ AdaptiveBatch::AdaptiveBatch(const pramaan_lp* lps, int count, const pramaan_pdh
     if (!opt_.refine) { xl_.alloc(n_); yl_.alloc(m_); }
     xsum_.alloc(n_); ysum_.alloc(m_); xm64_.alloc(n_); ym64_.alloc(m_); actm64_.alloc(m_); rcm64_.alloc(n_);
     rcon_.alloc(size_t(m_) * 4); ccon_.alloc(size_t(n_) * 4);
-    chunk_out_.alloc(size_t(std::max(rseg_.chunks, cseg_.chunks)) * 4 + 4);
+    chunk_out_.alloc(size_t(rseg_.chunks + cseg_.chunks) * 12 + 4);   // six reductions, three a side
     lp_out_.alloc(size_t(K_) * kOutWidth);
     action_.alloc(K_); inv_.alloc(K_); keep_.alloc(K_); dscale_.alloc(K_); pscale_.alloc(K_); lp_f_.alloc(K_);
     if (halpern_) {
@@ -560,8 +604,8 @@ AdaptiveBatch::AdaptiveBatch(const pramaan_lp* lps, int count, const pramaan_pdh
         set_int_kernel<<<1, 1, 0, st_>>>(iter_base_.get(), 0);
         PB_CUDA_CHECK(cudaGetLastError());
     }
-    tune_products();
     if (cluster_ok_) build_cluster_lps();
+    tune_products();
     PB_CUDA_CHECK(cudaStreamSynchronize(st_));
     // the packed host CSR stays for compaction
     h_rp_ = std::move(rp);
@@ -573,6 +617,7 @@ AdaptiveBatch::~AdaptiveBatch() {
     if (st_) cudaStreamSynchronize(st_);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (graph_) cudaGraphDestroy(graph_);
+    clear_resident();
     DeviceSyncScope gate;
     if (h_action_) cudaFreeHost(h_action_);
     if (h_restart_iter_) cudaFreeHost(h_restart_iter_);
@@ -604,20 +649,23 @@ void AdaptiveBatch::build_segments(Segments& s, const std::vector<int>& seg_begi
     PB_CUDA_CHECK(cudaStreamSynchronize(st_));   // host vectors are freed on return
 }
 
-void AdaptiveBatch::reduce(const Segments& s, const double* contrib, int width, bool max_op, int out_off) {
-    if (s.chunks > 0) {
-        if (max_op)
-            chunk_reduce_kernel<true><<<s.chunks, 256, 0, st_>>>(contrib, width, s.begin.get(), chunk_out_.get());
-        else
-            chunk_reduce_kernel<false><<<s.chunks, 256, 0, st_>>>(contrib, width, s.begin.get(), chunk_out_.get());
+void AdaptiveBatch::reduce(std::initializer_list<Reduction> list, bool max_op) {
+    ReduceJobs jobs{};
+    int chunks = 0;
+    for (const Reduction& r : list) {
+        jobs.job[jobs.n++] = ReduceJob{r.contrib, r.side->begin.get(), r.side->lp_first.get(), r.side->chunks, r.width,
+                                       r.out_off, chunks};
+        chunks += r.side->chunks;
     }
-    const int threads = K_ * width;
-    if (max_op)
-        lp_reduce_kernel<true><<<(threads + 255) / 256, 256, 0, st_>>>(chunk_out_.get(), width, s.lp_first.get(), K_,
-                                                                      lp_out_.get(), out_off);
-    else
-        lp_reduce_kernel<false><<<(threads + 255) / 256, 256, 0, st_>>>(chunk_out_.get(), width, s.lp_first.get(), K_,
-                                                                       lp_out_.get(), out_off);
+    if (chunk_out_.size() < size_t(chunks) * 4) chunk_out_.alloc(size_t(chunks) * 4);
+    if (chunks > 0) {
+        if (max_op) chunk_reduce_kernel<true><<<chunks, 256, 0, st_>>>(jobs, chunk_out_.get());
+        else chunk_reduce_kernel<false><<<chunks, 256, 0, st_>>>(jobs, chunk_out_.get());
+        PB_CUDA_CHECK(cudaGetLastError());
+    }
+    const int threads = jobs.n * K_ * 4;
+    if (max_op) lp_reduce_kernel<true><<<(threads + 255) / 256, 256, 0, st_>>>(jobs, chunk_out_.get(), K_, lp_out_.get());
+    else lp_reduce_kernel<false><<<(threads + 255) / 256, 256, 0, st_>>>(jobs, chunk_out_.get(), K_, lp_out_.get());
     PB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -691,7 +739,7 @@ void AdaptiveBatch::estimate_step_sizes() {
         SpmvLauncher<EpiStoreScaled, float, float, false>::launch(AT_.view(false), u.get(), e2, status_.get(), st_, dev_);
         dot2_contrib_kernel<<<grid_1d(n_), kThreads, 0, st_>>>(v.get(), w.get(), n_, ccon_.get());
         PB_CUDA_CHECK(cudaGetLastError());
-        reduce(cseg_, ccon_.get(), 2, false, 0);
+        reduce({{&cseg_, ccon_.get(), 2, 0}}, false);
         fetch_out();
         bool all = true;
         for (int q = 0; q < K_; ++q) {
@@ -878,7 +926,98 @@ void AdaptiveBatch::build_cluster_lps() {
     }
     cluster_size_ = C;
     cluster_auto_ = cluster_auto_ && C >= kClusterAutoMin;
-    if (use_cluster_kernel()) build_cluster_long_rows(v);
+    build_resident();
+    if (use_cluster_kernel() && resident_.empty()) build_cluster_long_rows(v);
+}
+
+void AdaptiveBatch::clear_resident() {
+    for (ResidentGroup& g : resident_) {
+        if (g.done) cudaEventDestroy(g.done);
+        if (g.stream) cudaStreamDestroy(g.stream);   // the batch waits for st_, which joins them
+    }
+    resident_.clear();
+    if (resident_ready_) cudaEventDestroy(resident_ready_);
+    resident_ready_ = nullptr;
+}
+
+void AdaptiveBatch::build_resident() {
+    clear_resident();
+    std::vector<int> lps;
+    std::vector<int4> shapes;
+    for (int q = 0; q < K_; ++q) {
+        const Lp& t = lp_[q];
+        if (!t.active || (t.r1 == t.r0 && t.c1 == t.c0)) continue;
+        lps.push_back(q);
+        shapes.push_back(make_int4(t.r1 - t.r0, t.c1 - t.c0, int(t.nnz), 0));
+    }
+    const std::vector<int> size = ResidentPlan::sizes_for(shapes, device_sm_count(dev_));
+    // All clusters side by side, or the tiled products run every LP: in two
+    // rounds the clusters are no faster (rolling-horizon LPs, us per iteration,
+    // clusters against tiled products: 2 LPs 2.4 / 8.1, 12 LPs 9.8 / 23.8, 24 LPs
+    // in 171 blocks 17.8 / 23.4, 32 LPs in 215 blocks 25.0 / 27.5, 128 LPs 85 / 61).
+    if (!ResidentPlan::side_by_side(size, device_sm_count(dev_))) return;
+    for (int s = kResMaxCluster + 1; s > 0; --s) {   // the largest clusters are launched first
+        ResidentGroup g;
+        std::vector<int4> ranges;
+        for (size_t k = 0; k < lps.size(); ++k) {
+            if (size[k] != (s > kResMaxCluster ? kResLean : s)) continue;
+            const Lp& t = lp_[lps[k]];
+            g.lps.push_back(lps[k]);
+            ranges.push_back(make_int4(t.r0, t.r1, t.c0, t.c1));
+        }
+        if (g.lps.empty()) continue;
+        g.active.assign(g.lps.size(), 1);
+        g.plan.build(A_, AT_, ranges, s > kResMaxCluster ? kResLean : s, st_);
+        if (use_cluster_kernel()) g.plan.prepare<ResHalpern<kResFlat>>();
+        else g.plan.prepare<ResHalpern<kResTiled>>();
+        const bool ok = g.plan.ok();
+        if (ok && !resident_.empty()) {
+            PB_CUDA_CHECK(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
+            PB_CUDA_CHECK(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));
+        }
+        resident_.push_back(std::move(g));
+        if (!ok) {
+            clear_resident();
+            return;
+        }
+    }
+    if (resident_.size() > 1) PB_CUDA_CHECK(cudaEventCreateWithFlags(&resident_ready_, cudaEventDisableTiming));
+}
+
+void AdaptiveBatch::launch_resident(int k) {
+    for (ResidentGroup& g : resident_) {
+        bool changed = false;
+        for (size_t i = 0; i < g.lps.size(); ++i) {
+            const char on = lp_[g.lps[i]].active ? 1 : 0;
+            changed = changed || on != g.active[i];
+            g.active[i] = on;
+        }
+        if (changed) g.plan.run_only(g.active, st_);
+    }
+    const int* lpr = K_ == 1 ? nullptr : lp_row_.get();
+    const int* lpc = K_ == 1 ? nullptr : lp_col_.get();
+    auto go = [&](auto algo) {
+        algo.x = x_.get(); algo.x_bar = xbar_.get(); algo.y = y_.get();
+        algo.tau = tau_.get(); algo.c = c_.get(); algo.l_x = lx_.get(); algo.u_x = ux_.get();
+        algo.sigma = sigma_.get(); algo.r_lo = lr_.get(); algo.r_hi = ur_.get(); algo.y_m = ym32_.get();
+        algo.lp_row = lpr; algo.lp_col = lpc;
+        algo.restart_iter = restart_iter_.get(); algo.iter_base = iter_base_.get();
+        algo.fpr_c0 = fpr_c_[0].get(); algo.fpr_c1 = fpr_c_[1].get();
+        algo.fpr_r0 = fpr_r_[0].get(); algo.fpr_r1 = fpr_r_[1].get();
+        algo.since = 0;
+        if (resident_ready_) PB_CUDA_CHECK(cudaEventRecord(resident_ready_, st_));
+        for (ResidentGroup& g : resident_) {
+            if (g.stream) PB_CUDA_CHECK(cudaStreamWaitEvent(g.stream, resident_ready_, 0));
+            g.plan.launch(A_, AT_, algo, k, status_.get(), g.stream ? g.stream : st_);
+        }
+        for (ResidentGroup& g : resident_) {
+            if (!g.stream) continue;
+            PB_CUDA_CHECK(cudaEventRecord(g.done, g.stream));
+            PB_CUDA_CHECK(cudaStreamWaitEvent(st_, g.done, 0));
+        }
+    };
+    if (use_cluster_kernel()) go(ResHalpern<kResFlat>{});
+    else go(ResHalpern<kResTiled>{});
 }
 
 void AdaptiveBatch::build_cluster_long_rows(const std::vector<int4>& lps) {
@@ -960,7 +1099,9 @@ void AdaptiveBatch::iterate(int k, int iter) {
         set_int_kernel<<<1, 1, 0, st_>>>(iter_base_.get(), iter);
         PB_CUDA_CHECK(cudaGetLastError());
     }
-    if (use_cluster_kernel()) {
+    if (!resident_.empty()) {
+        launch_resident(k);
+    } else if (use_cluster_kernel()) {
         launch_cluster(k);
     } else if (use_interval_kernel()) {
         launch_interval(k);
@@ -1003,7 +1144,7 @@ void AdaptiveBatch::materialize_average() {
     PB_CUDA_CHECK(cudaGetLastError());
 }
 
-void AdaptiveBatch::kkt(std::vector<KktSums>& cur, std::vector<KktSums>& avg, bool with_average) {
+void AdaptiveBatch::kkt(std::vector<KktSums>& cur, std::vector<KktSums>& avg, bool with_average, bool fpr) {
     if (with_average) materialize_average();
     const float* xs[2] = {x_.get(), xa_.get()};
     const float* ys[2] = {y_.get(), ya_.get()};
@@ -1013,11 +1154,20 @@ void AdaptiveBatch::kkt(std::vector<KktSums>& cur, std::vector<KktSums>& avg, bo
         if (m_ > 0) {
             EpiRowKktOut er{rlo64_.get(), rhi64_.get(), actm64_.get(), ym64_.get(), ys[k], rcon_.get()};
             launch_any<EpiRowKktOut, double, float>(A_, xs[k], er, status_.get(), st_, dev_);
-            reduce(rseg_, rcon_.get(), 4, false, 8 * k);
         }
         EpiColKktOut ec{cmin64_.get(), vlo64_.get(), vhi64_.get(), rcm64_.get(), xm64_.get(), xs[k], ccon_.get()};
         launch_any<EpiColKktOut, double, float>(AT_, ys[k], ec, status_.get(), st_, dev_);
-        reduce(cseg_, ccon_.get(), 4, false, 8 * k + 4);
+        const Reduction row{&rseg_, rcon_.get(), 4, 8 * k}, col{&cseg_, ccon_.get(), 4, 8 * k + 4};
+        if (fpr) {
+            // fixed-point residual of the interval's first and last iteration (slots 8-11)
+            const Reduction c0{&cseg_, fpr_c_[0].get(), 1, 8}, c1{&cseg_, fpr_c_[1].get(), 1, 10};
+            if (m_ > 0) reduce({row, col, c0, c1, {&rseg_, fpr_r_[0].get(), 1, 9}, {&rseg_, fpr_r_[1].get(), 1, 11}}, false);
+            else reduce({col, c0, c1}, false);
+        } else if (m_ > 0) {
+            reduce({row, col}, false);
+        } else {
+            reduce({col}, false);
+        }
     }
     fetch_out();
     cur.resize(size_t(K_));
@@ -1188,12 +1338,12 @@ void AdaptiveBatch::solve(const pramaan_lp* lps, pramaan_solve_result* results) 
                 dist_contrib_kernel<<<grid_1d(n_), kThreads, 0, st_>>>(x_.get(), refine ? nullptr : xl_.get(),
                                                                        cscale_.get(), n_, ccon_.get());
                 PB_CUDA_CHECK(cudaGetLastError());
-                reduce(cseg_, ccon_.get(), 1, false, 0);
+                reduce({{&cseg_, ccon_.get(), 1, 0}}, false);
                 if (m_) {
                     dist_contrib_kernel<<<grid_1d(m_), kThreads, 0, st_>>>(y_.get(), refine ? nullptr : yl_.get(),
                                                                            rscale_.get(), m_, rcon_.get());
                     PB_CUDA_CHECK(cudaGetLastError());
-                    reduce(rseg_, rcon_.get(), 1, false, 1);
+                    reduce({{&rseg_, rcon_.get(), 1, 1}}, false);
                 }
                 fetch_out();
                 for (int q = 0; q < K_; ++q) {
@@ -1270,15 +1420,7 @@ void AdaptiveBatch::solve_halpern() {
         const int chunk = std::min(cf, max_it - iter);
         iterate(chunk, iter);
         iter += chunk;
-        kkt(cur, avg, false);
-        // fixed-point residual of the interval's first and last iteration (slots 8-11)
-        reduce(cseg_, fpr_c_[0].get(), 1, false, 8);
-        reduce(cseg_, fpr_c_[1].get(), 1, false, 10);
-        if (m_) {
-            reduce(rseg_, fpr_r_[0].get(), 1, false, 9);
-            reduce(rseg_, fpr_r_[1].get(), 1, false, 11);
-        }
-        fetch_out();
+        kkt(cur, avg, false, /*fpr=*/true);
         bool any_restart = false, steps_changed = false, restart_changed = false;
         for (int q = 0; q < K_; ++q) {
             Lp& s = lp_[q];
@@ -1327,12 +1469,12 @@ void AdaptiveBatch::solve_halpern() {
             dist_contrib_kernel<<<grid_1d(n_), kThreads, 0, st_>>>(x_.get(), refine ? nullptr : xl_.get(),
                                                                    cscale_.get(), n_, ccon_.get());
             PB_CUDA_CHECK(cudaGetLastError());
-            reduce(cseg_, ccon_.get(), 1, false, 0);
+            reduce({{&cseg_, ccon_.get(), 1, 0}}, false);
             if (m_) {
                 dist_contrib_kernel<<<grid_1d(m_), kThreads, 0, st_>>>(y_.get(), refine ? nullptr : yl_.get(),
                                                                        rscale_.get(), m_, rcon_.get());
                 PB_CUDA_CHECK(cudaGetLastError());
-                reduce(rseg_, rcon_.get(), 1, false, 1);
+                reduce({{&rseg_, rcon_.get(), 1, 1}}, false);
             }
             fetch_out();
             for (int q = 0; q < K_; ++q) {
@@ -1486,8 +1628,8 @@ void AdaptiveBatch::compact() {
     graph_iters_ = 0;
     compacted_ = true;
     ++compactions_;
-    tune_products();
     if (cluster_ok_) build_cluster_lps();
+    tune_products();
 }
 
 // The launch autotuner on the current operands.  In Halpern mode it times the
@@ -1498,6 +1640,7 @@ void AdaptiveBatch::compact() {
 void AdaptiveBatch::tune_products() {
     // the iteration's vectors: steps, bounds, master and correction iterates, LP indices
     mark_l2_resident(A_, AT_, 32.0 * m_ + 36.0 * n_, dev_);
+    if (!resident_.empty()) return;   // the iteration launches no tiled product
     if (!halpern_) {
         autotune_operand(A_, st_, dev_, status_.get(), opt_.gather_cache, {}, 0, opt_.launch_blocks);
         autotune_operand(AT_, st_, dev_, status_.get(), opt_.gather_cache, {}, 0, opt_.launch_blocks);
@@ -1553,11 +1696,11 @@ void AdaptiveBatch::finish(const pramaan_lp* lps, pramaan_solve_result* results,
             launch_any<EpiStore<double, double>, double, double>(A, x_out_.get(), e, status_.get(), st_, dev_);
             EpiRowViolOut rv{rlo.get(), rhi.get(), rcon_.get()};
             launch_any<EpiRowViolOut, double, double>(A, x_out_.get(), rv, status_.get(), st_, dev_);
-            reduce(rs, rcon_.get(), 2, true, 0);
+            reduce({{&rs, rcon_.get(), 2, 0}}, true);
         }
         EpiColResidOut cr{x_out_.get(), c32.get(), vlo.get(), vhi.get(), opt_.tolerance, ccon_.get()};
         launch_any<EpiColResidOut, double, double>(AT, y_out_.get(), cr, status_.get(), st_, dev_);
-        reduce(cs, ccon_.get(), 3, true, 2);
+        reduce({{&cs, ccon_.get(), 3, 2}}, true);
         fetch_out();
         hx.resize(size_t(N));
         hy.resize(size_t(M));

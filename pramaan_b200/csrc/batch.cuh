@@ -27,10 +27,12 @@
 // iterates with FP32 corrections.
 #pragma once
 
+#include <initializer_list>
 #include <vector>
 
 #include "csr_device.cuh"
 #include "epilogues.cuh"
+#include "resident.cuh"
 
 namespace pb {
 
@@ -81,8 +83,14 @@ private:
     struct KktSums { double pr2, dr2, dobj, pobj; bool bad; };
 
     void build_segments(Segments& s, const std::vector<int>& seg_begin);
-    // per-LP sums (or maxima) of `width` interleaved contributions per element
-    void reduce(const Segments& s, const double* contrib, int width, bool max_op, int out_off);
+    // per-LP sums (or maxima) of `width` interleaved contributions per element,
+    // up to six arrays at a time
+    struct Reduction {
+        const Segments* side;
+        const double* contrib;
+        int width, out_off;
+    };
+    void reduce(std::initializer_list<Reduction> list, bool max_op);
     void fetch_out();
     void preconditioned_steps();
     void estimate_step_sizes();
@@ -92,7 +100,8 @@ private:
     // iteration j of an interval of k (Halpern mode writes the fixed-point
     // residual on the first and the last one)
     void iterate_once(int j, int k);
-    void kkt(std::vector<KktSums>& cur, std::vector<KktSums>& avg, bool with_average);
+    // `fpr`: the interval's fixed-point residuals as well (output slots 8-11)
+    void kkt(std::vector<KktSums>& cur, std::vector<KktSums>& avg, bool with_average, bool fpr = false);
     // Halpern mode on small operands: one cooperative kernel per check interval
     bool use_interval_kernel() const;
     void launch_interval(int k);
@@ -105,6 +114,11 @@ private:
     // the long-row lists of the cluster kernel for the LPs `lps` ({r0, r1, c0, c1})
     void build_cluster_long_rows(const std::vector<int4>& lps);
     void launch_cluster(int k);
+    // Halpern mode, LPs that fit a cluster's shared memory: the interval runs
+    // from there (resident.cuh), in the order of the sums of the path it
+    // stands for (the cluster kernel or the tiled products).
+    void build_resident();
+    void launch_resident(int k);
     void solve_halpern();
     void materialize_average();
     void push_actions();
@@ -158,6 +172,17 @@ private:
     bool cluster_ok_ = false;                // flat operands kept, cluster kernel allowed
     bool cluster_auto_ = false;              // every LP small enough for the automatic choice
     int cluster_nlps_ = 0, cluster_size_ = 1;
+    // One group of LPs per cluster size; the groups run side by side.
+    struct ResidentGroup {
+        ResidentPlan plan;
+        std::vector<int> lps;                // LP of every plan entry
+        std::vector<char> active;            // the ones the plan launches now
+        cudaStream_t stream = nullptr;       // null: st_
+        cudaEvent_t done = nullptr;
+    };
+    std::vector<ResidentGroup> resident_;    // empty: the other paths run
+    cudaEvent_t resident_ready_ = nullptr;
+    void clear_resident();
     DevBuf<int4> cluster_lps_;               // {r0, r1, c0, c1} per LP of the current layout
     // rows of A and of A^T longer than kClusterLongRow, per LP of the current
     // layout (ranges {a0, a1, at0, at1} into the two lists)

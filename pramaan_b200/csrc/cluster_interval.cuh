@@ -28,36 +28,12 @@
 #pragma once
 
 #include "adaptive.cuh"
+#include "cluster.cuh"
 
 namespace pb {
 
 constexpr int kClusterThreads = 512;    // threads per block of the cluster kernel
 constexpr int kClusterMax = 16;         // largest cluster (non-portable size)
-
-struct FlatCsr {
-    const int* row_ptr;
-    const int* col;
-    const float* val;
-};
-
-__device__ __forceinline__ unsigned cluster_rank_in() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_blocks() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_index_x() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // Rows r_u = r0 + u * step (u < kRows, those below r_end) of a flat CSR
 // times x, into acc[u]: each row's entries in CSR order, one FMA each.  The

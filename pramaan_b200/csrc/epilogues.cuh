@@ -35,13 +35,14 @@ struct EpiDualRef {
     __device__ void prefetch(int i) const {
         prefetch_l2(sigma + i); prefetch_l2(l_r + i); prefetch_l2(u_r + i); prefetch_l2(y + i);
     }
-    __device__ void apply(State&, int i, float ax) const {
-        const float sig = sigma[i];
-        if (sig <= 0.0f) return;
-        const float w = __fadd_rn(__fdiv_rn(y[i], sig), ax);
-        const float wp = fminf(fmaxf(w, l_r[i]), u_r[i]);
-        y[i] = __fmul_rn(sig, __fsub_rn(w, wp));
+    // The new y of a row.
+    __device__ static float update(float y_old, float sig, float lo, float hi, float ax) {
+        if (sig <= 0.0f) return y_old;
+        const float w = __fadd_rn(__fdiv_rn(y_old, sig), ax);
+        const float wp = fminf(fmaxf(w, lo), hi);
+        return __fmul_rn(sig, __fsub_rn(w, wp));
     }
+    __device__ void apply(State&, int i, float ax) const { y[i] = update(y[i], sigma[i], l_r[i], u_r[i], ax); }
     __device__ void finish(State&, int) const {}
 };
 
@@ -63,12 +64,18 @@ struct EpiPrimalRef {
         prefetch_l2(tau + j); prefetch_l2(c + j); prefetch_l2(l_x + j); prefetch_l2(u_x + j);
         prefetch_l2(x + j);
     }
+    // The new x of a column, and its extrapolation in xb.
+    __device__ static float update(float x_prev, float t, float cost, float lo, float hi, float aty, float& xb) {
+        const float g = __fadd_rn(cost, aty);
+        const float step = __fmaf_rn(-t, g, x_prev);
+        const float x_new = fminf(fmaxf(step, lo), hi);
+        xb = __fmaf_rn(2.0f, x_new, -x_prev);
+        return x_new;
+    }
     __device__ void apply(State&, int j, float aty) const {
-        const float x_prev = x[j];
-        const float g = __fadd_rn(c[j], aty);
-        const float step = __fmaf_rn(-tau[j], g, x_prev);
-        const float x_new = fminf(fmaxf(step, l_x[j]), u_x[j]);
-        x_bar[j] = __fmaf_rn(2.0f, x_new, -x_prev);
+        float xb;
+        const float x_new = update(x[j], tau[j], c[j], l_x[j], u_x[j], aty, xb);
+        x_bar[j] = xb;
         x[j] = x_new;
     }
     __device__ void finish(State&, int) const {}

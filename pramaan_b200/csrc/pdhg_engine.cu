@@ -209,8 +209,16 @@ PdhgEngine::PdhgEngine(const pramaan_lp& lp, const pramaan_pdhg_options& opt) : 
         build_panel_split(A_, panel_, opt.panel_split, dev_, st_);
         build_panel_hot(A_, AT_, panel_, panel_t_, opt.gather_cache, dev_, st_);
     }
+    // Small LPs: the iterations run on one cluster, from the flat operands.
+    const int cluster = ResidentPlan::sizes_for({make_int4(m_, n_, lp.nnz, 0)}, device_sm_count(dev_))[0];
+    const bool small = !adaptive_ && !panel_.active && m_ > 0 && n_ > 0 && lp.nnz > 0 && cluster != 0;
+    A_.keep_flat = AT_.keep_flat = small;
     A_.pack(st_);
     AT_.pack(st_);
+    if (small) {
+        resident_.build(A_, AT_, {make_int4(0, m_, 0, n_)}, cluster, st_);
+        resident_.prepare<ResReference>();
+    }
     // the iteration's vectors: sigma, bounds, y (rows); tau, c, bounds, x, x̄ (columns), plus the gathers
     mark_l2_resident(A_, AT_, 20.0 * m_ + 28.0 * n_, dev_);
     // Occupancy queries / smem attributes before any graph capture.
@@ -428,6 +436,12 @@ void PdhgEngine::build_graph(int k) {
 
 void PdhgEngine::iterate(int k) {
     if (k <= 0) return;
+    if (resident_.ok() && !opt_.profile_kernels) {
+        const ResReference algo{x_.get(),  xbar_.get(), y_.get(),  tau_.get(), c_.get(), lx_.get(),
+                                ux_.get(), sigma_.get(), lr_.get(), ur_.get(), nullptr};
+        resident_.launch(A_, AT_, algo, k, status_.get(), st_);
+        return;
+    }
     const bool graph = opt_.use_graph && !opt_.profile_kernels && k <= 4096;
     if (graph) {
         if (graph_iters_ != k) build_graph(k);

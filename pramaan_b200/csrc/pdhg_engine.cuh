@@ -6,6 +6,7 @@
 #include "csr_device.cuh"
 #include "epilogues.cuh"
 #include "panel.cuh"
+#include "resident.cuh"
 
 namespace pb {
 
@@ -122,6 +123,7 @@ private:
     CsrDevice A_, AT_;
     PanelSplit panel_;   // A x̄ over column panels (reference mode, power-law operands)
     PanelHot panel_t_;   // the longest rows' part of Aᵀy over the same panels
+    ResidentPlan resident_;   // small LPs (reference mode): iterations on one cluster
     DevBuf<float> c_, lr_, ur_, lx_, ux_, sigma_, tau_, x_, y_, xbar_;
     DevBuf<double> rlo64_, rhi64_, vlo64_, vhi64_, slots_;
     DevBuf<int> status_;
