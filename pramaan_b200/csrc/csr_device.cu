@@ -118,7 +118,7 @@ __device__ int row_of_entry(const int* __restrict__ rp_c, int rows_c, long long 
     return lo;
 }
 
-// meta[t] = {first_row, tail_continues, 0, 0}
+// meta[t] = {first_row, tail_continues, rows ending, 0}
 //   first_row      compacted row holding the tile's first entry
 //   tail_continues 1 when the row holding the tile's last entry continues into
 //                  the next tile
@@ -132,7 +132,7 @@ __global__ void meta_kernel(const int* __restrict__ rp_c, int rows_c, int tiles,
         const int tr = row_of_entry(rp_c, rows_c, last);
         const long long tend = rp_c[tr + 1];
         const int cont = (tr < rows_c && tend > last + 1) ? 1 : 0;
-        meta[t] = make_int4(fr, cont, 0, 0);
+        meta[t] = make_int4(fr, cont, min(cont ? tr : tr + 1, rows_c) - fr, 0);
         begins[t] = (cont && rp_c[tr] >= base) ? 1 : 0;
     }
 }
@@ -204,6 +204,121 @@ __global__ void pack_kernel(const int* __restrict__ col, const float* __restrict
         }
         for (int k = threadIdx.x; k < FW; k += blockDim.x) rf[k] = flags[size_t(t) * FW + k];
         if (threadIdx.x == 0) *reinterpret_cast<int4*>(r + TileRec::off_meta) = meta[t];
+    }
+}
+
+// ---- row-aligned tiles -------------------------------------------------------
+// The rows are cut into segments of about kAlignSegment entries; a warp per
+// segment fills tiles with whole rows, looking at 256 rows a step (one round
+// trip; 32 rows a step took three times as long on rows of 4 entries).  A row
+// that does not fit the rest of a tile starts the next one, unless it is longer
+// than a tile: such a row follows on and crosses.
+constexpr int kAlignSegment = 64 * kSpmvTile;
+constexpr int kAlignLook = 8;
+
+struct AlignedTile { int first_entry, entries, first_row, ending, continues; };
+
+__device__ int first_row_at(const int* __restrict__ rp_c, int rows_c, long long entry) {
+    int lo = 0, hi = rows_c;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rp_c[mid] >= entry) hi = mid; else lo = mid + 1;
+    }
+    return lo;
+}
+
+// Pass 1 (tiles == nullptr): tiles and crossing rows of every segment.
+// Pass 2: the tiles from tile_at[s] on, and the crossing rows from cross_at[s] - cross_at[0] on.
+__global__ void align_kernel(const int* __restrict__ rp_c, const int* __restrict__ row_map, int rows_c, int segments,
+                             int* __restrict__ n_tiles, int* __restrict__ n_cross, const int* __restrict__ tile_at,
+                             const int* __restrict__ cross_at, AlignedTile* __restrict__ tiles,
+                             int4* __restrict__ cross) {
+    constexpr int T = kSpmvTile;
+    const int s = int((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (s >= segments) return;
+    int r = first_row_at(rp_c, rows_c, (long long)s * kAlignSegment);
+    const int r_end = s == segments - 1 ? rows_c : first_row_at(rp_c, rows_c, (s + 1LL) * kAlignSegment);
+    const int t0 = tiles ? tile_at[s] : 0, x0 = tiles ? cross_at[s] - cross_at[0] : 0;
+    int t = 0, x = 0;
+    int e0 = r < r_end ? rp_c[r] : 0, first = r;
+    auto emit = [&](int entries, int ending, int continues) {
+        if (tiles && lane == 0) tiles[t0 + t] = AlignedTile{e0, entries, first, ending, continues};
+        ++t;
+    };
+    while (r < r_end) {
+        int end[kAlignLook], fits = 0;
+#pragma unroll
+        for (int u = 0; u < kAlignLook; ++u) end[u] = rp_c[min(r + 32 * u + lane, r_end - 1) + 1];
+#pragma unroll
+        for (int u = 0; u < kAlignLook; ++u)
+            fits += __popc(__ballot_sync(0xffffffffu, r + 32 * u + lane < r_end && end[u] - e0 <= T));
+        r += fits;
+        if (fits == 32 * kAlignLook || r >= r_end) continue;
+        const int begin = rp_c[r], stop = rp_c[r + 1];
+        if (stop - begin <= T) {
+            emit(begin - e0, r - first, 0);
+            e0 = begin;
+            first = r;
+            continue;
+        }
+        const int opens = t;   // the tile the long row begins in
+        if (begin - e0 == T) { // which is full already: the next one
+            emit(T, r - first, 0);
+            e0 = begin;
+            first = r;
+        }
+        const int at = begin - e0 == 0 ? t : opens;
+        while (stop - e0 > T) {
+            emit(T, r - first, 1);
+            e0 += T;
+            first = r;
+        }
+        if (tiles && lane == 0) cross[x0 + x] = make_int4(row_map ? row_map[r] : r, t0 + at, t - at + 1, 0);
+        ++x;
+        ++r;
+    }
+    if (first < r_end) emit(rp_c[r_end] - e0, r_end - first, 0);
+    if (!tiles && lane == 0) {
+        n_tiles[s] = t;
+        n_cross[s] = x;
+    }
+}
+
+// One block per row-aligned tile: its record and its slab of remainders.
+__global__ void __launch_bounds__(256) pack_aligned_kernel(
+    const int* __restrict__ col, const float* __restrict__ val, const float* __restrict__ lo,
+    const int* __restrict__ rp_c, const int* __restrict__ slot, const AlignedTile* __restrict__ tiles, int num_tiles,
+    unsigned char* __restrict__ rec, float* __restrict__ lo_out) {
+    constexpr int TW = TileRec::TW, FW = TileRec::FW;
+    __shared__ uint32_t bits[FW];
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        const AlignedTile d = tiles[t];
+        unsigned char* r = rec + size_t(t) * TileRec::bytes;
+        int* rc = reinterpret_cast<int*>(r + TileRec::off_col);
+        float* rv = reinterpret_cast<float*>(r + TileRec::off_val);
+        if (threadIdx.x < FW) bits[threadIdx.x] = 0u;
+        __syncthreads();
+        for (int k = threadIdx.x; k < TW; k += blockDim.x) {
+            const bool in = k < d.entries;
+            int c = in ? col[size_t(d.first_entry) + k] : 0;
+            if (in && slot) {
+                const int h = slot[c];
+                if (h >= 0) c = ~h;
+            }
+            rc[tile_slot(k)] = c;
+            rv[tile_slot(k)] = in ? val[size_t(d.first_entry) + k] : 0.0f;
+            if (lo_out) lo_out[size_t(t) * TW + tile_slot(k)] = in ? lo[size_t(d.first_entry) + k] : 0.0f;
+        }
+        // row starts; row first_row + ending starts at the padding, or is the one that continues
+        for (int i = threadIdx.x; i <= d.ending; i += blockDim.x) {
+            const int q = rp_c[d.first_row + i] - d.first_entry;
+            if (q >= 0 && q < TW) atomicOr(&bits[q >> 5], 1u << (q & 31));
+        }
+        __syncthreads();
+        if (threadIdx.x < FW) reinterpret_cast<uint32_t*>(r + TileRec::off_flags)[threadIdx.x] = bits[threadIdx.x];
+        if (threadIdx.x == 0)
+            *reinterpret_cast<int4*>(r + TileRec::off_meta) = make_int4(d.first_row, d.continues, d.ending, 0);
+        __syncthreads();
     }
 }
 
@@ -399,7 +514,9 @@ void select_hot_pair(CsrDevice& A, CsrDevice& AT, int dev, cudaStream_t st) {
 
 void CsrDevice::pack(cudaStream_t st) {
     if (packed) return;
-    if (num_tiles > 0) {
+    if (num_tiles > 0 && align_rows && pack_aligned(st)) {
+        // (records, crossing rows and remainders replaced)
+    } else if (num_tiles > 0) {
         rec.alloc(size_t(num_tiles) * TileRec::bytes);
         const int grid = num_tiles < 65535 * 4 ? num_tiles : 65535 * 4;
         pack_kernel<<<grid, 256, 0, st>>>(col.get(), val.get(), flags.get(), meta.get(),
@@ -422,7 +539,57 @@ void CsrDevice::pack(cudaStream_t st) {
     }
     flags.reset();
     meta.reset();
+    rp_c.reset();
     packed = true;
+}
+
+bool CsrDevice::pack_aligned(cudaStream_t st) {
+    const int segments = ceil_div(nnz, kAlignSegment), len = segments + 1;
+    const long long most =
+        std::min((long long)(0x7fffffff / kSpmvTile), (long long)((1.0 + align_rows_max) * num_tiles) + 1);   // nnz_pad
+    // One scratch buffer: the segments' counts (tiles, then crossing rows), their offsets, the tiles' list.
+    size_t tb = 0;
+    PB_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, tb, (int*)nullptr, (int*)nullptr, 2 * len, st));
+    const size_t list_at = (size_t(16) * len + tb + 15) & ~size_t(15);
+    DevBuf<unsigned char> scratch(list_at + size_t(most) * sizeof(AlignedTile));
+    int* counts = reinterpret_cast<int*>(scratch.get());
+    int* at = counts + 2 * len;
+    AlignedTile* tiles = reinterpret_cast<AlignedTile*>(scratch.get() + list_at);
+    PB_CUDA_CHECK(cudaMemsetAsync(counts, 0, size_t(8) * len, st));
+    const int* map = num_empty > 0 ? row_map.get() : nullptr;
+    const int grid = ceil_div(segments, kThreads / 32);
+    align_kernel<<<grid, kThreads, 0, st>>>(rp_c.get(), map, rows_c, segments, counts, counts + len, nullptr, nullptr,
+                                            nullptr, nullptr);
+    PB_CUDA_CHECK(cudaGetLastError());
+    PB_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(scratch.get() + size_t(16) * len, tb, counts, at, 2 * len, st));
+    int sums[2] = {0, 0};   // tiles; tiles and crossing rows
+    PB_CUDA_CHECK(cudaMemcpyAsync(&sums[0], at + len, 4, cudaMemcpyDeviceToHost, st));
+    PB_CUDA_CHECK(cudaMemcpyAsync(&sums[1], at + 2 * len - 1, 4, cudaMemcpyDeviceToHost, st));
+    PB_CUDA_CHECK(cudaStreamSynchronize(st));
+    const int count = sums[0], crossing = sums[1] - count;
+    if (count > most) return false;
+    if (crossing > num_cross) cross.alloc(size_t(crossing));
+    align_kernel<<<grid, kThreads, 0, st>>>(rp_c.get(), map, rows_c, segments, nullptr, nullptr, at, at + len, tiles,
+                                            cross.get());
+    PB_CUDA_CHECK(cudaGetLastError());
+    if (count > num_tiles) {
+        carry.alloc(size_t(2) * count);
+        PB_CUDA_CHECK(cudaMemsetAsync(carry.get(), 0, carry.bytes(), st));
+    }
+    num_tiles = count;
+    nnz_pad = count * kSpmvTile;
+    num_cross = crossing;
+    aligned = true;
+    rec.alloc(size_t(count) * TileRec::bytes);
+    const bool lo = has_lo && val_lo.get();
+    DevBuf<float> lo_i(lo ? size_t(nnz_pad) : 0);
+    pack_aligned_kernel<<<std::min(count, 65535 * 4), 256, 0, st>>>(col.get(), val.get(), lo ? val_lo.get() : nullptr,
+                                                                   rp_c.get(), hot > 0 ? hot_slot.get() : nullptr,
+                                                                   tiles, count, rec.get(), lo_i.get());
+    PB_CUDA_CHECK(cudaGetLastError());
+    PB_CUDA_CHECK(cudaStreamSynchronize(st));   // the scratch is freed on return
+    if (lo) val_lo = std::move(lo_i);
+    return true;
 }
 
 void CsrDevice::allocate(int rows_, int cols_, int nnz_, bool lo) {
@@ -473,7 +640,7 @@ void CsrDevice::finalize(cudaStream_t st) {
         row_map.reset();
         empty_rows.reset();
     }
-    DevBuf<int> rp_c(size_t(rows_c) + 2);
+    rp_c.alloc(size_t(rows_c) + 2);
     if (rows > 0) {
         compact_rows_kernel<<<grid_1d(rows), kThreads, 0, st>>>(
             row_ptr.get(), ne.get(), idx.get(), rows, rp_c.get(), num_empty > 0 ? row_map.get() : nullptr,

@@ -8,7 +8,7 @@
 //                                      both lane-interleaved (tile_slot),
 //                                      flags u32[16] (bit q: entry q starts a
 //                                      non-empty row), meta int4
-//                                      {first_row, tail_continues, 0, 0}
+//                                      {first_row, tail_continues, rows ending, 0}
 //   val_lo     fp32  [nnz_pad]         FP32(value - val), kept only when some
 //                                      value is not exactly representable (entry
 //                                      order while building, tile_slot order
@@ -99,8 +99,11 @@ public:
     int l2_resident = 0;           // keep the records in L2 between launches (see mark_l2_resident)
     bool has_lo = false;
     bool packed = false;
+    bool align_rows = false;       // pack() starts a row that fits one tile in one tile (see align_rows_max)
+    bool aligned = false;          // pack() did so; the tile kernel takes the empty rows as well
     bool keep_flat = false;        // pack() keeps the flat col / val (FP32) arrays
                                    // for kernels that read the plain CSR
+    DevBuf<int> rp_c;              // non-empty rows' first entries, then nnz and nnz_pad (until pack())
     DevBuf<int> row_ptr, col, row_map, empty_rows, hot_idx, hot_slot;
     DevBuf<float> val, val_lo;
     DevBuf<uint32_t> flags;
@@ -111,7 +114,8 @@ public:
     CsrView view(bool with_lo) const {
         CsrView v;
         v.rows = rows; v.cols = cols; v.nnz = nnz; v.nnz_pad = nnz_pad; v.num_tiles = num_tiles;
-        v.rows_c = rows_c; v.num_empty = num_empty; v.num_cross = num_cross;
+        v.rows_c = rows_c; v.num_cross = num_cross;
+        (aligned ? v.tile_empty : v.num_empty) = num_empty;
         v.blocks_per_sm = tuned_blocks_per_sm;
         if (!packed && num_tiles > 0) throw std::logic_error("CsrDevice::view before pack()");
         v.rec = rec.get();
@@ -135,6 +139,13 @@ public:
     void allocate(int rows_, int cols_, int nnz_, bool lo);
     // Builds flags / meta / row compaction / crossing rows from row_ptr.
     void finalize(cudaStream_t st);
+    // Row-aligned tiles are taken when they add at most this share of tiles (the
+    // records are the traffic: a share more of them costs about that share of a
+    // product, and the fixup launch they save is 6 to 10 % of a product of 4 to 26
+    // million non-zeros, more of smaller ones).  us per reference iteration, cut |
+    // row-aligned: uniform 0.4 M non-zeros 17.1 | 10.8, uniform 4 M 49.0 | 43.8,
+    // banded 1 M 12.2 | 8.4, banded 26 M 101.2 | 92.9.
+    static constexpr double align_rows_max = 0.08;
     // Interleaves col / val / flags / meta into tile records and frees them
     // (entries whose target has a hot slot get ~slot).
     void pack(cudaStream_t st);
@@ -146,6 +157,9 @@ public:
     // loads every slot once); the slots are kept only when they take at least
     // kSpmvHotMinShare of the non-zeros.  No-op for small operands.
     void select_hot(const int* target_rp, int num_targets, int dev, cudaStream_t st);
+    // The records with row-aligned tiles; false (and nothing changed) when they
+    // would take too many.
+    bool pack_aligned(cudaStream_t st);
     size_t device_bytes() const {
         return row_ptr.bytes() + col.bytes() + row_map.bytes() + empty_rows.bytes() + hot_idx.bytes() +
                val.bytes() + val_lo.bytes() + flags.bytes() + meta.bytes() + cross.bytes() +

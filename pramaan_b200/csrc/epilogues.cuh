@@ -42,7 +42,11 @@ struct EpiDualRef {
         const float wp = fminf(fmaxf(w, lo), hi);
         return __fmul_rn(sig, __fsub_rn(w, wp));
     }
-    __device__ void apply(State&, int i, float ax) const { y[i] = update(y[i], sigma[i], l_r[i], u_r[i], ax); }
+    static constexpr bool kSplit = true;
+    struct In { float y, sig, lo, hi; };
+    __device__ In load(int i) const { return In{y[i], sigma[i], l_r[i], u_r[i]}; }
+    __device__ void store(State&, int i, const In& in, float ax) const { y[i] = update(in.y, in.sig, in.lo, in.hi, ax); }
+    __device__ void apply(State& st, int i, float ax) const { store(st, i, load(i), ax); }
     __device__ void finish(State&, int) const {}
 };
 
@@ -72,12 +76,16 @@ struct EpiPrimalRef {
         xb = __fmaf_rn(2.0f, x_new, -x_prev);
         return x_new;
     }
-    __device__ void apply(State&, int j, float aty) const {
+    static constexpr bool kSplit = true;
+    struct In { float x, t, c, lo, hi; };
+    __device__ In load(int j) const { return In{x[j], tau[j], c[j], l_x[j], u_x[j]}; }
+    __device__ void store(State&, int j, const In& in, float aty) const {
         float xb;
-        const float x_new = update(x[j], tau[j], c[j], l_x[j], u_x[j], aty, xb);
+        const float x_new = update(in.x, in.t, in.c, in.lo, in.hi, aty, xb);
         x_bar[j] = xb;
         x[j] = x_new;
     }
+    __device__ void apply(State& st, int j, float aty) const { store(st, j, load(j), aty); }
     __device__ void finish(State&, int) const {}
 };
 
@@ -93,7 +101,13 @@ struct EpiPrimalRefAdd {
         base.prefetch(j);
         prefetch_l2(add + j);
     }
-    __device__ void apply(State& s, int j, float aty) const { base.apply(s, j, __fadd_rn(add[j], aty)); }
+    static constexpr bool kSplit = true;
+    struct In { EpiPrimalRef::In base; float add; };
+    __device__ In load(int j) const { return In{base.load(j), add[j]}; }
+    __device__ void store(State& s, int j, const In& in, float aty) const {
+        base.store(s, j, in.base, __fadd_rn(in.add, aty));
+    }
+    __device__ void apply(State& s, int j, float aty) const { store(s, j, load(j), aty); }
     __device__ void finish(State&, int) const {}
 };
 

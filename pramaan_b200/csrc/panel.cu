@@ -524,6 +524,7 @@ void build_panel_split(const CsrDevice& A, PanelSplit& ps, int mode, int dev, cu
     // ---- the short rows as their own operand ----
     CsrDevice& S = ps.S;
     S.allocate(rows, cols, ns, /*lo=*/false);
+    S.align_rows = true;
     PB_CUDA_CHECK(cudaMemcpyAsync(S.row_ptr.get(), s_rp.get(), (size_t(rows) + 1) * 4, cudaMemcpyDeviceToDevice, st));
     if (ns > 0) {
         short_copy_kernel<<<grid_for_n(rows), kThreads, 0, st>>>(A.row_ptr.get(), A.col.get(), A.val.get(),
@@ -697,6 +698,7 @@ void build_panel_hot(const CsrDevice& A, const CsrDevice& AT, const PanelSplit& 
     DevBuf<float> hval{size_t(nhot)};
     CsrDevice& R = ph.rest;
     R.allocate(cols, rows, nrest, /*lo=*/false);
+    R.align_rows = true;
     PB_CUDA_CHECK(cudaMemcpyAsync(R.row_ptr.get(), roff.get(), (size_t(cols) + 1) * 4, cudaMemcpyDeviceToDevice, st));
     split_copy_kernel<<<grid_for_n(cols), kThreads, 0, st>>>(AT.row_ptr.get(), AT.col.get(), AT.val.get(), cols,
                                                             hot.get(), hidx.get(), hoff.get(), roff.get(), hcol.get(),

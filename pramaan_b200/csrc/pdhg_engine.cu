@@ -211,8 +211,10 @@ PdhgEngine::PdhgEngine(const pramaan_lp& lp, const pramaan_pdhg_options& opt) : 
     }
     // Small LPs: the iterations run on one cluster, from the flat operands.
     const int cluster = ResidentPlan::sizes_for({make_int4(m_, n_, lp.nnz, 0)}, device_sm_count(dev_))[0];
-    const bool small = !adaptive_ && !panel_.active && m_ > 0 && n_ > 0 && lp.nnz > 0 && cluster != 0;
+    const bool small = !adaptive_ && !panel_.active && m_ > 0 && n_ > 0 && lp.nnz > 0 && cluster != 0 &&
+                       !opt.profile_kernels;
     A_.keep_flat = AT_.keep_flat = small;
+    A_.align_rows = AT_.align_rows = !adaptive_ && !small;
     A_.pack(st_);
     AT_.pack(st_);
     if (small) {
@@ -436,7 +438,7 @@ void PdhgEngine::build_graph(int k) {
 
 void PdhgEngine::iterate(int k) {
     if (k <= 0) return;
-    if (resident_.ok() && !opt_.profile_kernels) {
+    if (resident_.ok()) {
         const ResReference algo{x_.get(),  xbar_.get(), y_.get(),  tau_.get(), c_.get(), lx_.get(),
                                 ux_.get(), sigma_.get(), lr_.get(), ur_.get(), nullptr};
         resident_.launch(A_, AT_, algo, k, status_.get(), st_);
