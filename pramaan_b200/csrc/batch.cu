@@ -951,11 +951,14 @@ void AdaptiveBatch::build_resident() {
         shapes.push_back(make_int4(t.r1 - t.r0, t.c1 - t.c0, int(t.nnz), 0));
     }
     const std::vector<int> size = ResidentPlan::sizes_for(shapes, device_sm_count(dev_));
-    // All clusters side by side, or the tiled products run every LP: in two
-    // rounds the clusters are no faster (rolling-horizon LPs, us per iteration,
-    // clusters against tiled products: 2 LPs 2.4 / 8.1, 12 LPs 9.8 / 23.8, 24 LPs
-    // in 171 blocks 17.8 / 23.4, 32 LPs in 215 blocks 25.0 / 27.5, 128 LPs 85 / 61).
-    if (!ResidentPlan::side_by_side(size, device_sm_count(dev_))) return;
+    // Clusters for every LP, or the tiled products run them all (those also run
+    // a batch with an LP that no cluster holds).  Rolling-horizon LPs, us per
+    // iteration, clusters against tiled products: 2 LPs 2.4 | 8.1, 16 LPs (0.9
+    // rounds) 8.0 | 24.4, 32 LPs (1.6) 16.0 | 27.7, 32 LPs (2.2) 19.2 | 31.0, 48 LPs
+    // (2.9) 22.8 | 33.5, 64 LPs (4.1) 35.9 | 55.3, 128 LPs (8.2) 77 | 86.  A round
+    // costs 8 to 10 us whatever follows it, the tiled products their fixed 20 to 25
+    // us once, so beyond that they catch up.
+    if (ResidentPlan::rounds(size, device_sm_count(dev_)) > ResidentPlan::kMaxRounds) return;
     for (int s = kResMaxCluster + 1; s > 0; --s) {   // the largest clusters are launched first
         ResidentGroup g;
         std::vector<int4> ranges;

@@ -7,13 +7,15 @@ namespace pb {
 
 namespace {
 
-// First row r of [r0, r1] whose rows before it weigh at least `share` of the
-// LP: shared-memory bytes of a row, 8 per entry and 28 for its own vectors.
+// First row r of [r0, r1] whose rows before it weigh at least `part` of `parts`
+// of the LP, an entry 2 and a row 1.  (By shared-memory bytes, 8 and 28, the
+// blocks with a planning LP's coupling rows, 48 entries each at the end of A,
+// had 190 of them, the largest share of memory and twice the others' time.)
 __device__ int share_begin(const int* __restrict__ rp, int r0, int r1, int part, int parts) {
     if (part == 0) return r0;
     if (part == parts) return r1;
     const long long base = rp[r0];
-    auto weight = [&](int r) { return 8 * ((long long)rp[r] - base) + 28LL * (r - r0); };
+    auto weight = [&](int r) { return 2 * ((long long)rp[r] - base) + (r - r0); };
     const long long want = weight(r1) * part / parts;
     int lo = r0, hi = r1;
     while (lo < hi) {
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(256) slot_kernel(ResCta* __restrict__ cta, int
         const int len = r < n ? rp[begin + r + 1] - rp[begin + r] : 0;
         const int lines = __reduce_max_sync(0xffffffffu, len <= kResLongRow ? len : 0);
         const int count = __popc(__ballot_sync(0xffffffffu, len > kResLongRow));
-        const int entries = __reduce_add_sync(0xffffffffu, len > kResLongRow ? len : 0);
+        const int entries = __reduce_add_sync(0xffffffffu, len > kResLongRow ? res_long_stride(len) : 0);
         if (lane == 0) {
             own_lines[s] = uint32_t(lines);
             if (count) {
@@ -138,18 +140,13 @@ bool ResidentPlan::cut(const CsrDevice& A, const CsrDevice& AT, const std::vecto
     std::vector<ResCta> h(static_cast<size_t>(blocks));
     PB_CUDA_CHECK(cudaMemcpyAsync(h.data(), cta_.get(), h.size() * sizeof(ResCta), cudaMemcpyDeviceToHost, st));
     PB_CUDA_CHECK(cudaStreamSynchronize(st));
-    need_x_ = need_y_ = 0;
-    for (const ResCta& c : h) {
-        need_x_ = std::max(need_x_, c.need_x);
-        need_y_ = std::max(need_y_, c.need_y);
-    }
-    if (std::max(need_x_, need_y_) * kResSub > 65536) return false;   // positions are 16 bits
     smem_ = 0;
     for (const ResCta& c : h) {
+        if (std::max(c.need_x, c.need_y) * kResSub > 65536) return false;   // positions are 16 bits
         // before the layout's byte counts, which are ints
         const long long entries = 32LL * c.ell_a + 32LL * c.ell_t + c.lent_a + c.lent_t;
         if (8 * entries > (long long)kResMaxSmem) return false;
-        smem_ = std::max(smem_, size_t(ResLayout(c, need_x_, need_y_, size, lean_).total));
+        smem_ = std::max(smem_, size_t(ResLayout(c, size, lean_).total));
     }
     return smem_ <= kResMaxSmem;
 }
@@ -180,23 +177,23 @@ std::vector<int> ResidentPlan::sizes_for(const std::vector<int4>& shapes, int sm
         std::vector<int> larger = size;
         for (size_t k = 0; k < size.size(); ++k) {
             const int subs = (std::max(shapes[k].x, shapes[k].y) + kResSub - 1) / kResSub;
-            if (size[k] > 0 && size[k] < kResMaxCluster && 4 * subs > 3 * size[k] * (kResThreads / 32))
+            if (size[k] > 0 && size[k] < kResMaxCluster && 4 * subs > 3 * size[k] * 16)
                 larger[k] = next_size(size[k]);
         }
-        if (larger == size || !side_by_side(larger, sms)) return size;
+        if (larger == size || rounds(larger, sms) > 1.0) return size;
         size = std::move(larger);
     }
 }
 
 // A cluster lies in one GPC, of 18 to 20 SMs: the largest take a GPC each (7 at
 // a time on 148 SMs).
-bool ResidentPlan::side_by_side(const std::vector<int>& sizes, int sms) {
+double ResidentPlan::rounds(const std::vector<int>& sizes, int sms) {
     long long taken = 0;
     for (int s : sizes) {
-        if (s == 0) return false;
+        if (s == 0) return 1e30;
         taken += s == kResLean || s == kResMaxCluster ? 20 : s == 8 ? 9 : s;
     }
-    return taken <= sms;
+    return double(taken) / sms;
 }
 
 void ResidentPlan::build(const CsrDevice& A, const CsrDevice& AT, const std::vector<int4>& lps, int size,

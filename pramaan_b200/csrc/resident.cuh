@@ -69,6 +69,10 @@ constexpr int kResWeights = 128;       // iterations whose weights are computed 
 constexpr int kResLongRow = 16;
 constexpr int kResFlat = 0, kResTiled = 1;
 constexpr uint16_t kResNoSlot = 0xffff;
+// Entries a long row takes: 2 modulo 16, so that the 8 rows a warp sums at a
+// time begin in different banks (rows of 48 back to back all began in the same
+// one: a block with 130 of them took 4,300 cycles for its half, 3,200 now).
+__host__ __device__ constexpr int res_long_stride(int len) { return len + ((2 - len) & 15); }
 constexpr size_t kResMaxSmem = 232448;
 
 // One block's share (rows of A, columns of A) and what it receives.
@@ -89,15 +93,14 @@ struct ResView {
     int sub_x = 0, sub_y = 0;
     const uint32_t* lines_a = nullptr;  // [block][sub_y]: first line of an own sub-chunk << 5 | lines
     const uint32_t* lines_t = nullptr;
-    int max_need_x = 0, max_need_y = 0;
     FlatCsr A{}, AT{};
     const uint16_t* idx_a = nullptr;    // positions of the entries' columns in the own gather vector
     const uint16_t* idx_t = nullptr;
     int* status = nullptr;
 };
 
-// Shared memory of one block.  The gather vectors come first, at the same
-// place in every block of the launch: senders address them.
+// Shared memory of one block.  The gather vectors come first, where senders
+// find them: x̄'s at kGather, y's behind the sub-chunks of x̄ the block needs.
 struct ResLayout {
     static constexpr int kBarX = 0, kBarY = 8, kCounts = 16, kWeights = 128, kGather = kWeights + 4 * kResWeights;
     int gx, gy, sx, sy, cols, rows, x, long_sum, ell_a, ell_t, lent_a, lent_t, range_a, range_t, lines_a, lines_t, long_a,
@@ -105,7 +108,7 @@ struct ResLayout {
     int total;
     int R, C;
     // lean: the elements' constants stay in global memory
-    __host__ __device__ ResLayout(const ResCta& c, int max_need_x, int max_need_y, int cluster, bool lean) {
+    __host__ __device__ ResLayout(const ResCta& c, int cluster, bool lean) {
         R = c.r1 - c.r0;
         C = c.c1 - c.c0;
         int at = kGather;
@@ -115,8 +118,8 @@ struct ResLayout {
             return p;
         };
         const int subs_x = (C + kResSub - 1) / kResSub, subs_y = (R + kResSub - 1) / kResSub;
-        gx = take(max_need_x * kResSub * 4);
-        gy = take(max_need_y * kResSub * 4);
+        gx = take(c.need_x * kResSub * 4);
+        gy = take(c.need_y * kResSub * 4);
         sx = take(subs_x * kResSub * 4);           // own x̄ (before: sums of long columns)
         sy = take(subs_y * kResSub * 4);           // own y
         cols = take(lean ? 0 : C * 16);            // {tau, c, lower, upper}
@@ -502,7 +505,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResView 
     const int first_cta = (v.which ? v.which[cluster_index_x()] : int(cluster_index_x())) * cluster;
     const int my_cta = first_cta + int(cluster_rank_in());
     const ResCta me = v.cta[my_cta];
-    const ResLayout L(me, v.max_need_x, v.max_need_y, cluster, kLean);
+    const ResLayout L(me, cluster, kLean);
     const int R = L.R, C = L.C;
     uint64_t* bar_x = reinterpret_cast<uint64_t*>(smem + ResLayout::kBarX);
     uint64_t* bar_y = reinterpret_cast<uint64_t*>(smem + ResLayout::kBarY);
@@ -548,7 +551,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResView 
             const bool far = len > kResLongRow;
             int at = 0;
             if (far) {
-                at = atomicAdd(entries, len);
+                at = atomicAdd(entries, res_long_stride(len));
                 longs[atomicAdd(listed, 1)] = make_int4(r, at, len, b);
             }
             unsigned todo = __ballot_sync(0xffffffffu, far);
@@ -593,6 +596,9 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResView 
         }
     }
     // the receivers of every own sub-chunk
+    const uint32_t gather_x = smem_u32(smem) + ResLayout::kGather;   // of block `lane` of the cluster
+    const uint32_t gather_y =
+        gather_x + (lane < cluster ? unsigned(v.cta[first_cta + lane].need_x) * (kResSub * 4) : 0u);
     auto find_receivers = [&](const uint16_t* slots, int stride, int first, int n, uint32_t gather, uint64_t* bar,
                               uint2* to, uint8_t* count) {
         for (int s = warp; s < n; s += kWarps) {
@@ -604,8 +610,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResView 
             if (lane == 0) count[s] = uint8_t(__popc(m));
         }
     };
-    find_receivers(v.slot_x, v.sub_x, (me.c0 - me.lc0) / kResSub, subs_x, smem_u32(gx), bar_x, to_x, n_to_x);
-    find_receivers(v.slot_y, v.sub_y, (me.r0 - me.lr0) / kResSub, subs_y, smem_u32(gy), bar_y, to_y, n_to_y);
+    find_receivers(v.slot_x, v.sub_x, (me.c0 - me.lc0) / kResSub, subs_x, gather_x, bar_x, to_x, n_to_x);
+    find_receivers(v.slot_y, v.sub_y, (me.r0 - me.lr0) / kResSub, subs_y, gather_y, bar_y, to_y, n_to_y);
     algo.begin(me);
     __syncthreads();
     const int nlong_a = counts[0], nlong_t = counts[1];
@@ -748,8 +754,10 @@ public:
     // kResLean: the largest clusters with the constants in global memory;
     // 0: too large for any cluster.
     static std::vector<int> sizes_for(const std::vector<int4>& shapes, int sms);
-    // Whether clusters of these sizes run at the same time (false with a size 0).
-    static bool side_by_side(const std::vector<int>& sizes, int sms);
+    // How often over clusters of these sizes fill the SMs (1 or less: they run
+    // at the same time; infinite with a size 0).
+    static constexpr double kMaxRounds = 8.0;
+    static double rounds(const std::vector<int>& sizes, int sms);
 
     // Cuts the LPs {r0, r1, c0, c1} over clusters of `size` blocks, or of the
     // next size that holds them all.  Leaves ok() false when none does.
@@ -773,8 +781,6 @@ public:
         v.lines_t = lines_t_.get();
         v.sub_x = sub_x_;
         v.sub_y = sub_y_;
-        v.max_need_x = need_x_;
-        v.max_need_y = need_y_;
         v.A = fa;
         v.AT = ft;
         v.idx_a = idx_a_.get();
@@ -823,7 +829,7 @@ private:
     bool cut(const CsrDevice& A, const CsrDevice& AT, const std::vector<int4>& lps, int size, cudaStream_t st);
 
     bool lean_ = false;
-    int clusters_ = 0, running_ = 0, size_ = 1, sub_x_ = 0, sub_y_ = 0, need_x_ = 0, need_y_ = 0;
+    int clusters_ = 0, running_ = 0, size_ = 1, sub_x_ = 0, sub_y_ = 0;
     size_t smem_ = 0;
     DevBuf<int4> lps_;
     DevBuf<int> which_;

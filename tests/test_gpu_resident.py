@@ -91,3 +91,17 @@ def test_reference_iteration_against_fp64(shape):
     ox, oy, _ = oracle.trajectory(md, k)
     assert np.allclose(gx, ox, rtol=1e-4, atol=1e-4)
     assert np.allclose(gy, oy, rtol=1e-4, atol=1e-4 * (1 + abs(oy).max()))
+
+
+def test_more_clusters_than_fit_at_once_and_the_largest_lps():
+    """Several rounds of clusters, an LP that fits only without its constants in
+    shared memory, and coupling rows at the end of A (a block of long rows)."""
+    rng = np.random.default_rng(8)
+    shapes = [(336, 50), (300, 46), (260, 48), (170, 33)] * 2 + [(60, 20), (24, 5)] * 6
+    models = [rolling_horizon_lp(T, P, rng=rng) for T, P in shapes]
+    o = dict(tolerance=0.0, max_iterations=130, check_frequency=64, algorithm=ALGO_HALPERN)
+    a = solve_batch(models, PdhgOptions(persistent=0, **o))
+    b = solve_batch(models, PdhgOptions(persistent=-1, **o))
+    for p, q in zip(a, b):
+        assert p.iterations == q.iterations and p.restarts == q.restarts
+        assert np.array_equal(p.x, q.x) and np.array_equal(p.y, q.y)
