@@ -709,28 +709,96 @@ static void check_structure(int* d_flag, cudaStream_t st) {
     if (h & 2) throw InvalidArgument("col_idx entry out of bounds");
 }
 
-void csr_upload_f64(CsrDevice& A, int rows, int cols, int nnz, const int* h_row_ptr,
-                    const int* h_col, const double* h_val, cudaStream_t st, int* d_flag) {
-    A.allocate(rows, cols, nnz, /*lo=*/true);
-    upload_structure(A, rows, cols, nnz, h_row_ptr, h_col, st, d_flag);
-    check_structure(d_flag, st);
+// FP64 values in v64 -> FP32 hi / lo, then the row structure.  Synchronises st.
+static void split_values(CsrDevice& A, int nnz, const DevBuf<double>& v64, cudaStream_t st) {
     if (nnz > 0) {
-        DevBuf<double> v64{size_t(nnz)};
         DevBuf<int> inexact(1);
         PB_CUDA_CHECK(cudaMemsetAsync(inexact.get(), 0, 4, st));
-        PB_CUDA_CHECK(cudaMemcpyAsync(v64.get(), h_val, size_t(nnz) * 8, cudaMemcpyHostToDevice, st));
         split_f64_kernel<<<grid_1d(nnz), kThreads, 0, st>>>(v64.get(), nnz, A.val.get(),
                                                             A.val_lo.get(), inexact.get());
         PB_CUDA_CHECK(cudaGetLastError());
         int h_inexact = 0;
         PB_CUDA_CHECK(cudaMemcpyAsync(&h_inexact, inexact.get(), 4, cudaMemcpyDeviceToHost, st));
-        PB_CUDA_CHECK(cudaStreamSynchronize(st));   // v64 freed below
+        PB_CUDA_CHECK(cudaStreamSynchronize(st));
         if (!h_inexact) { A.val_lo.reset(); A.has_lo = false; }
     } else {
         A.val_lo.reset();
         A.has_lo = false;
     }
     A.finalize(st);
+}
+
+void csr_upload_f64(CsrDevice& A, int rows, int cols, int nnz, const int* h_row_ptr,
+                    const int* h_col, const double* h_val, cudaStream_t st, int* d_flag) {
+    A.allocate(rows, cols, nnz, /*lo=*/true);
+    upload_structure(A, rows, cols, nnz, h_row_ptr, h_col, st, d_flag);
+    check_structure(d_flag, st);
+    DevBuf<double> v64{size_t(nnz)};
+    if (nnz > 0)
+        PB_CUDA_CHECK(cudaMemcpyAsync(v64.get(), h_val, size_t(nnz) * 8, cudaMemcpyHostToDevice, st));
+    split_values(A, nnz, v64, st);
+}
+
+// Rows and entries of packed LPs: the LP's own row pointers and columns become
+// the packed ones.  at[k] = {first row, first entry, first column, columns}.
+// Flag bit 2: a column outside its LP.
+__global__ void shift_parts_kernel(int* __restrict__ row_ptr, int* __restrict__ col, const int4* __restrict__ at,
+                                   int parts, int rows, int nnz, int* __restrict__ flag) {
+    PB_GRID_STRIDE(i, (long long)rows + nnz + 1) {
+        if (i == rows) {
+            row_ptr[rows] = nnz;
+            continue;
+        }
+        const bool row = i < rows;
+        const int q = int(row ? i : i - rows - 1);
+        int lo = 0, hi = parts - 1;   // the last part that begins at or before q
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if ((row ? at[mid].x : at[mid].y) <= q) lo = mid; else hi = mid - 1;
+        }
+        const int4 p = at[lo];
+        if (row) {
+            row_ptr[q] = int((long long)row_ptr[q] + p.y);
+        } else {
+            const int c = col[q];
+            if (c < 0 || c >= p.w) atomicOr(flag, 2);
+            else col[q] = c + p.z;
+        }
+    }
+}
+
+void csr_upload_f64_parts(CsrDevice& A, int rows, int cols, int nnz, const std::vector<CsrPart>& parts, cudaStream_t st) {
+    A.allocate(rows, cols, nnz, /*lo=*/true);
+    DevBuf<double> v64{size_t(nnz)};
+    DevBuf<int> flag(1);
+    DevBuf<int4> at{parts.size()};
+    PB_CUDA_CHECK(cudaMemsetAsync(flag.get(), 0, 4, st));
+    std::vector<int4> first;
+    size_t r0 = 0, e0 = 0, c0 = 0;
+    for (const CsrPart& p : parts) {
+        first.push_back(make_int4(int(r0), int(e0), int(c0), p.cols));
+        if (p.rows > 0)
+            PB_CUDA_CHECK(cudaMemcpyAsync(A.row_ptr.get() + r0, p.row_ptr, size_t(p.rows) * 4, cudaMemcpyHostToDevice, st));
+        if (p.nnz > 0) {
+            PB_CUDA_CHECK(cudaMemcpyAsync(A.col.get() + e0, p.col, size_t(p.nnz) * 4, cudaMemcpyHostToDevice, st));
+            PB_CUDA_CHECK(cudaMemcpyAsync(v64.get() + e0, p.val, size_t(p.nnz) * 8, cudaMemcpyHostToDevice, st));
+        }
+        r0 += size_t(p.rows);
+        e0 += size_t(p.nnz);
+        c0 += size_t(p.cols);
+    }
+    PB_CUDA_CHECK(cudaMemcpyAsync(at.get(), first.data(), first.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    shift_parts_kernel<<<grid_1d((long long)rows + nnz + 1), kThreads, 0, st>>>(A.row_ptr.get(), A.col.get(), at.get(),
+                                                                              int(parts.size()), rows, nnz, flag.get());
+    validate_kernel<<<grid_1d((long long)rows + nnz + 1), kThreads, 0, st>>>(A.row_ptr.get(), A.col.get(), rows, cols,
+                                                                           nnz, flag.get());
+    PB_CUDA_CHECK(cudaGetLastError());
+    int h = 0;
+    PB_CUDA_CHECK(cudaMemcpyAsync(&h, flag.get(), 4, cudaMemcpyDeviceToHost, st));
+    PB_CUDA_CHECK(cudaStreamSynchronize(st));
+    if (h & 2) throw InvalidArgument("pramaan_lp: col_idx entry out of bounds");
+    if (h & 1) throw InvalidArgument("row_ptr must start at 0, be non-decreasing and end at nnz");
+    split_values(A, nnz, v64, st);
 }
 
 void csr_upload_f32(CsrDevice& A, int rows, int cols, int nnz, const int* h_row_ptr,

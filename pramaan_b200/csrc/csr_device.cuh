@@ -170,6 +170,12 @@ public:
 // Uploads a host CSR with FP64 values (reference ModelIR layout) and splits
 // every value into FP32 hi + FP32 lo on the device.  `d_flag` receives a
 // nonzero code when row_ptr is not monotone or a column index is out of range.
+// csr_upload_f64 of a block-diagonal operand whose blocks (one or more, in order)
+// lie in the caller's arrays: each goes to its place on the device and the
+// device shifts its row pointers and columns.  Throws InvalidArgument for a
+// column outside its block or row pointers that do not form one CSR.
+struct CsrPart { const int* row_ptr; const int* col; const double* val; int rows, cols, nnz; };
+void csr_upload_f64_parts(CsrDevice& A, int rows, int cols, int nnz, const std::vector<CsrPart>& parts, cudaStream_t st);
 void csr_upload_f64(CsrDevice& A, int rows, int cols, int nnz, const int* h_row_ptr,
                     const int* h_col, const double* h_val, cudaStream_t st, int* d_flag);
 // Uploads a host CSR with FP32 values (test-harness launchers).
