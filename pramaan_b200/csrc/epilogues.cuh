@@ -43,6 +43,7 @@ struct EpiDualRef {
         return __fmul_rn(sig, __fsub_rn(w, wp));
     }
     static constexpr bool kSplit = true;
+    static constexpr int kAhead = 2;
     struct In { float y, sig, lo, hi; };
     __device__ In load(int i) const { return In{y[i], sigma[i], l_r[i], u_r[i]}; }
     __device__ void store(State&, int i, const In& in, float ax) const { y[i] = update(in.y, in.sig, in.lo, in.hi, ax); }
@@ -77,6 +78,7 @@ struct EpiPrimalRef {
         return x_new;
     }
     static constexpr bool kSplit = true;
+    static constexpr int kAhead = 2;
     struct In { float x, t, c, lo, hi; };
     __device__ In load(int j) const { return In{x[j], tau[j], c[j], l_x[j], u_x[j]}; }
     __device__ void store(State&, int j, const In& in, float aty) const {
@@ -102,6 +104,7 @@ struct EpiPrimalRefAdd {
         prefetch_l2(add + j);
     }
     static constexpr bool kSplit = true;
+    static constexpr int kAhead = 2;
     struct In { EpiPrimalRef::In base; float add; };
     __device__ In load(int j) const { return In{base.load(j), add[j]}; }
     __device__ void store(State& s, int j, const In& in, float aty) const {

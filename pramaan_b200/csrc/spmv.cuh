@@ -216,21 +216,22 @@ struct SpmvSmemLayout {
 
 // Epilogues that split apply() into load(row) -> In and store(State&, row,
 // In, value) declare `static constexpr bool kSplit = true`; the tile loop then
-// loads the first kEpiAhead rows per lane while the tile's gathers are in
-// flight, and kEpiPass rows per lane ahead of their updates after that.  (All
+// loads kEpiPass rows per lane ahead of their updates, and with `static
+// constexpr int kAhead` the first kAhead rows per lane while the tile's gathers
+// are in flight.  (All
 // warps of an SM gather and update at about the same time, so an update's
 // round trip leaves the gather path idle.)  us per reference iteration, no row
-// ahead | two: uniform 4 M non-zeros 51.5 | 49.0, banded 26 M 102.8 | 101.2.
+// ahead | two: uniform 4 M non-zeros 51.5 | 49.0, banded 26 M 102.8 | 101.2.  The
+// Halpern updates have more inputs: with two rows ahead their kernels spill.
 template <class Epi, class = void>
 struct EpiSplit { static constexpr bool value = false; };
 template <class Epi>
 struct EpiSplit<Epi, decltype(void(Epi::kSplit))> { static constexpr bool value = Epi::kSplit; };
 constexpr int kEpiPass = 4;
-constexpr int kEpiAhead = 2;
-template <class Epi, bool kSplit = EpiSplit<Epi>::value>
-struct EpiIn { using type = typename Epi::In; };
+template <class Epi, class = void>
+struct EpiAhead { static constexpr int value = 0; struct In {}; };
 template <class Epi>
-struct EpiIn<Epi, false> { struct type {}; };
+struct EpiAhead<Epi, decltype(void(Epi::kAhead))> { static constexpr int value = Epi::kAhead; using In = typename Epi::In; };
 
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
@@ -403,19 +404,19 @@ __device__ __forceinline__ bool spmv_tiles(const CsrView& A, const XT* __restric
         const int skip = (s0 == 0 && meta.z > 0) ? 1 : 0;
         const int base = meta.x + skip;
         const int n_fin = meta.z - skip;   // without a virtual padding row
-        typename EpiIn<Epi>::type ahead[kEpiAhead];
-        int ahead_row[kEpiAhead];
-        if constexpr (EpiSplit<Epi>::value) {
+        constexpr int kAhead = EpiAhead<Epi>::value;
+        typename EpiAhead<Epi>::In ahead[kAhead > 0 ? kAhead : 1];
+        int ahead_row[kAhead > 0 ? kAhead : 1];
+        if constexpr (kAhead > 0) {
 #pragma unroll
-            for (int u = 0; u < kEpiAhead; ++u) {
+            for (int u = 0; u < kAhead; ++u) {
                 const int k = lane + 32 * u;
                 ahead_row[u] = k < n_fin ? (kRowMap ? A.row_map[base + k] : base + k) : -1;
                 if (ahead_row[u] >= 0) ahead[u] = epi.load(ahead_row[u]);
             }
         }
         if constexpr (!kRowMap) {
-            for (int k = (EpiSplit<Epi>::value ? 32 * kEpiAhead : 0) + lane * 8; k < n_fin; k += 256)
-                epi.prefetch(base + k);
+            for (int k = 32 * kAhead + lane * 8; k < n_fin; k += 256) epi.prefetch(base + k);
         }
 
         // ---- walk my entries; stage the rows that end here ----
@@ -479,11 +480,13 @@ __device__ __forceinline__ bool spmv_tiles(const CsrView& A, const XT* __restric
             // per lane are loaded before any of them is updated, so the loads
             // of a tile with many short rows overlap instead of running one
             // round trip per 32 rows.
+            if constexpr (kAhead > 0) {
 #pragma unroll
-            for (int u = 0; u < kEpiAhead; ++u)
-                if (ahead_row[u] >= 0) epi.store(est, ahead_row[u], ahead[u], fin[lane + 32 * u]);
+                for (int u = 0; u < kAhead; ++u)
+                    if (ahead_row[u] >= 0) epi.store(est, ahead_row[u], ahead[u], fin[lane + 32 * u]);
+            }
             constexpr int U = kEpiPass;
-            for (int k0 = 32 * kEpiAhead + lane; k0 < n_fin; k0 += 32 * U) {
+            for (int k0 = 32 * kAhead + lane; k0 < n_fin; k0 += 32 * U) {
                 typename Epi::In in[U];
                 int row[U];
 #pragma unroll
