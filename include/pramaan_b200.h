@@ -103,9 +103,13 @@ typedef struct pramaan_pdhg_options {
     double reserved_d;
     int32_t persistent;       /* Halpern mode, how a check interval runs:
                                  0 (default): one thread-block cluster per LP
-                                 runs the whole interval in one launch when
-                                 every LP has at most 2^20 non-zeros, else as -1;
-                                 2: the cluster kernel for any size;
+                                 runs the whole interval in one launch: from
+                                 its shared memory when every LP fits there
+                                 (about 50,000 variables) and the clusters fill
+                                 the GPU at most 8 times, else from L2 when the
+                                 LPs are few and have at most 2^20 non-zeros,
+                                 else as -1;
+                                 2: clusters for any size;
                                  1: one cooperative kernel over the packed
                                  operand (grid barriers between the products);
                                  -1: the two tiled products per iteration,

@@ -128,8 +128,9 @@ class PdhgOptions:
     use_graph: bool = True
     profile_kernels: bool = False
     refine: bool = True         # adaptive mode: FP64 master iterates + FP32 corrections
-    persistent: int = 0         # Halpern mode: 0 one cluster per LP runs each check interval when every LP
-                                # has <= 2^20 non-zeros (else -1), 2 the cluster kernel always,
+    persistent: int = 0         # Halpern mode: 0 one cluster per LP runs each check interval, from its
+                                # shared memory when every LP fits, else from L2 for few LPs of
+                                # <= 2^20 non-zeros (else -1), 2 clusters always,
                                 # 1 one cooperative kernel per interval, -1 two dependent launches
                                 # per iteration in a CUDA graph
     gather_cache: int = 0       # 0: hot gather targets of large skewed operands in shared memory and
