@@ -78,7 +78,7 @@ struct EpiPrimalRef {
         return x_new;
     }
     static constexpr bool kSplit = true;
-    static constexpr int kAhead = 2;
+    static constexpr int kAhead = 1;
     struct In { float x, t, c, lo, hi; };
     __device__ In load(int j) const { return In{x[j], tau[j], c[j], l_x[j], u_x[j]}; }
     __device__ void store(State&, int j, const In& in, float aty) const {
@@ -104,7 +104,7 @@ struct EpiPrimalRefAdd {
         prefetch_l2(add + j);
     }
     static constexpr bool kSplit = true;
-    static constexpr int kAhead = 2;
+    static constexpr int kAhead = 1;
     struct In { EpiPrimalRef::In base; float add; };
     __device__ In load(int j) const { return In{base.load(j), add[j]}; }
     __device__ void store(State& s, int j, const In& in, float aty) const {

@@ -221,8 +221,10 @@ struct SpmvSmemLayout {
 // are in flight.  (All
 // warps of an SM gather and update at about the same time, so an update's
 // round trip leaves the gather path idle.)  us per reference iteration, no row
-// ahead | two: uniform 4 M non-zeros 51.5 | 49.0, banded 26 M 102.8 | 101.2.  The
-// Halpern updates have more inputs: with two rows ahead their kernels spill.
+// ahead | two: uniform 4 M non-zeros 51.5 | 49.0, banded 26 M 102.8 | 101.2;
+// with one row in the primal update, whose kernel spilled with two, 43.2 and 84.8
+// (row-aligned tiles, two in both 44.0 and 93.0).  The Halpern updates have more
+// inputs still: none ahead.
 template <class Epi, class = void>
 struct EpiSplit { static constexpr bool value = false; };
 template <class Epi>
