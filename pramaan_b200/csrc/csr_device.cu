@@ -556,7 +556,9 @@ bool CsrDevice::pack_aligned(cudaStream_t st) {
     int* at = counts + 2 * len;
     AlignedTile* tiles = reinterpret_cast<AlignedTile*>(scratch.get() + list_at);
     PB_CUDA_CHECK(cudaMemsetAsync(counts, 0, size_t(8) * len, st));
-    const int* map = num_empty > 0 ? row_map.get() : nullptr;
+    // The rows are compacted whenever there is a map: num_empty may have been
+    // trimmed since finalize() (the panel split keeps only A's own empty rows).
+    const int* map = row_map.get();
     const int grid = ceil_div(segments, kThreads / 32);
     align_kernel<<<grid, kThreads, 0, st>>>(rp_c.get(), map, rows_c, segments, counts, counts + len, nullptr, nullptr,
                                             nullptr, nullptr);
