@@ -430,13 +430,11 @@ AdaptiveBatch::AdaptiveBatch(const pramaan_lp* lps, int count, const pramaan_pdh
     K_ = int(lp_.size());
     m_ = int(m); n_ = int(n); nnz_ = int(nnz);
     full_m_ = m_; full_n_ = n_;
-    PB_CUDA_CHECK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    PB_CUDA_CHECK(pinned_alloc(&h_status_, sizeof(int)));
-    status_.alloc(1);
-    PB_CUDA_CHECK(cudaMemsetAsync(status_.get(), 0, sizeof(int), st_));
-    if (K_ == 0) return;
 
     // ---- pack the LPs (host), minimisation form ----
+    // Every LP is checked by itself, before the device sees any: its rows must
+    // hold its own entries and these its own columns (the packed bounds, which
+    // the device checks, would let it reach into its neighbours).
     const size_t M = static_cast<size_t>(m_), N = static_cast<size_t>(n_), NZ = static_cast<size_t>(nnz_);
     std::vector<int> rp(M + 1), ci(NZ), lp_row(M), lp_col(N);
     std::vector<double> val(NZ), rl(M), ru(M), vl(N), vu(N), cmin(N);
@@ -469,10 +467,16 @@ AdaptiveBatch::AdaptiveBatch(const pramaan_lp* lps, int count, const pramaan_pdh
             rp[s.r0 + i] = int(e0 + lp.row_ptr[i]);
         }
         s.b_norm = std::sqrt(b2);
+        if (lp.num_rows > 0 ? lp.row_ptr[0] != 0 || lp.row_ptr[lp.num_rows] != lp.nnz : lp.nnz != 0)
+            throw InvalidArgument("pramaan_lp: row_ptr must start at 0, be non-decreasing and end at nnz");
+        unsigned last = 0;   // the largest column, a negative one above all others
         for (int k = 0; k < lp.nnz; ++k) {
-            ci[e0 + k] = lp.col_idx[k] + s.c0;
+            last = std::max(last, unsigned(lp.col_idx[k]));
+            ci[e0 + k] = int(unsigned(lp.col_idx[k]) + unsigned(s.c0));
             val[e0 + k] = lp.values[k];
         }
+        if (lp.nnz > 0 && last >= unsigned(lp.num_cols))
+            throw InvalidArgument("pramaan_lp: col_idx entry out of bounds");
         e0 += lp.nnz;
         rseg[q] = s.r0; cseg[q] = s.c0;
     }
@@ -499,6 +503,11 @@ AdaptiveBatch::AdaptiveBatch(const pramaan_lp* lps, int count, const pramaan_pdh
         }
     }
 
+    PB_CUDA_CHECK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
+    PB_CUDA_CHECK(pinned_alloc(&h_status_, sizeof(int)));
+    status_.alloc(1);
+    PB_CUDA_CHECK(cudaMemsetAsync(status_.get(), 0, sizeof(int), st_));
+    if (K_ == 0) return;
     PB_CUDA_CHECK(pinned_alloc(&h_action_, sizeof(int) * K_));
     PB_CUDA_CHECK(pinned_alloc(&h_inv_, sizeof(double) * K_));
     PB_CUDA_CHECK(pinned_alloc(&h_dscale_, sizeof(float) * K_));
