@@ -395,12 +395,14 @@ PRAMAAN_API int pramaan_launch_pdhg_iteration(float* h_x, float* h_y, const floa
  * graph, and hosts that own the device memory pool.  All pointers are device
  * pointers owned by the caller (row_ptr[m+1], col_idx[nnz], values[nnz], x[n],
  * y[m]); the work is queued on `stream` (a cudaStream_t, NULL for the legacy
- * default stream) and the call returns without waiting.  Partial sums of very
- * long rows (from 512 entries on) go to a 512 KiB scratch array compiled into the
- * library (a file-scope __device__ array, held by every GPU that loads the
- * library until exit), which limits nnz to 134,217,728; larger inputs are
- * rejected with PRAMAAN_ERR_INVALID_ARGUMENT.  Every call shares that array:
- * calls on one stream are ordered, calls that overlap on the GPU race.  The
+ * default stream) and the call returns without waiting.  A product of at most
+ * 16,384 non-zeros keeps everything on chip.  In a larger one the partial sums
+ * of very long rows (more than 512 entries) go to a 512 KiB scratch array
+ * compiled into the library (a file-scope __device__ array, held by every GPU
+ * that loads the library until exit), which limits nnz to 134,217,728; larger
+ * inputs are rejected with PRAMAAN_ERR_INVALID_ARGUMENT.  These products share
+ * that array: calls on one stream are ordered, and when two of them overlap on
+ * the GPU their very long rows race (other rows and smaller products do not).  The
  * first call on a device looks up the array's device address and caches it
  * for that device's primary context; it allocates nothing itself, but under
  * lazy module loading it is where the library's module, and with it the

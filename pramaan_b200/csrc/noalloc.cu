@@ -16,15 +16,18 @@
 // shared memory, then the rows of the tile summed by 1 to 8 lanes each, or by
 // the whole warp where a row is long).  Owning whole rows leaves nothing to
 // combine between warps, except for giant rows (more than 2 T entries): those
-// are cut at the range boundaries, every range sums its piece into the scratch
-// array below, and the pieces of a row are added in a fixed order afterwards:
-// by the same launch when the whole product fits one thread-block cluster
-// (nnz <= 16,384), else by a second, dependent one.  The scratch is the
-// file-scope array below: every GPU that loads the library holds it (512 KiB)
-// until the process exits, one call is limited to nnz <= 134,217,728, and
-// every call shares it, so calls that overlap on the GPU (on different
-// streams) race; calls on one stream are ordered.  Every slot a call reads is
-// written earlier in the same call, so nothing needs clearing between calls.
+// are cut at the range boundaries, every range leaves the sum of its piece, and
+// the pieces of a row are added in a fixed order afterwards.  A product that
+// fits one thread-block cluster (nnz <= 16,384) does so in the same launch and
+// keeps the pieces in the shared memory of the cluster's first block.  A larger
+// one keeps them in the scratch array below and adds them in a second,
+// dependent launch.  The scratch is a file-scope array: every GPU that loads
+// the library holds it (512 KiB) until the process exits, one call is limited
+// to nnz <= 134,217,728, and all larger products share it, so when two of them
+// overlap on the GPU (on different streams) the sums of their giant rows race;
+// calls on one stream are ordered.  What a call reads there it has written
+// itself, so nothing needs clearing between calls; a row number that another
+// call left there is checked against the call's own row_ptr before it is used.
 //
 // What bounds it: the gathers.  B200 serves random 4-byte gathers at about one
 // sector per SM per clock (ceiling.cu), 14 us for 4 M entries and 97 us for
@@ -245,9 +248,35 @@ __device__ __forceinline__ float row_sums(const float* __restrict__ p, int from,
     return sum;
 }
 
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Where the ranges leave their words: the scratch array, or the shared memory
+// of the cluster's first block.
+struct GlobalWords {
+    float* at;
+    __device__ __forceinline__ void ready() const {}
+    __device__ __forceinline__ void put(int i, float v) const { at[i] = v; }
+    __device__ __forceinline__ float get(int i) const { return __ldcg(at + i); }
+};
+struct ClusterWords {
+    float* own;       // this block's array (the first block's is the one in use)
+    uint32_t first;   // the first block's, as an address in the cluster
+    __device__ explicit ClusterWords(float* shared) : own(shared) {
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(first) : "r"(smem_u32(shared)));
+    }
+    __device__ __forceinline__ void ready() const { cluster_wait(); }   // the first block runs
+    __device__ __forceinline__ void put(int i, float v) const {
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(first + 4u * unsigned(i)), "f"(v) : "memory");
+    }
+    __device__ __forceinline__ float get(int i) const { return own[i]; }
+};
+
 // One range by one warp.
-template <bool kVec>
-__device__ __forceinline__ void range_product(const NaArgs& a, int k, int lane, float* __restrict__ p) {
+template <bool kVec, class Words>
+__device__ __forceinline__ void range_product(const NaArgs& a, const Words& words, int k, int lane, float* __restrict__ p) {
     const unsigned last_col = static_cast<unsigned>(a.n - 1);
     const bool last = k == a.ranges - 1;
     const int lo = k * a.T, hi = last ? a.nnz : lo + a.T;
@@ -259,11 +288,12 @@ __device__ __forceinline__ void range_product(const NaArgs& a, int k, int lane, 
     int e1 = r1 > r ? rp(r1) : 0;
     // ---- pieces of giant rows ----
     const int kGiant = 2 * a.T;
+    words.ready();
     if (r > 0) {
         const int s = rp(r - 1), e = r1 > r ? e0 : rp(r);
         if (e > lo && e - s > kGiant) {
             const float t = piece_sum(a, lo, min(e, hi), last_col, lane);
-            if (lane == 0) a.carry[kNaSlots * k] = t;
+            if (lane == 0) words.put(kNaSlots * k, t);
         }
     }
     int giant = -1;
@@ -272,11 +302,11 @@ __device__ __forceinline__ void range_product(const NaArgs& a, int k, int lane, 
         if (e1 - s > kGiant) {
             giant = --r1;
             const float t = piece_sum(a, s, min(e1, hi), last_col, lane);
-            if (lane == 0) a.carry[kNaSlots * k + 1] = t;
+            if (lane == 0) words.put(kNaSlots * k + 1, t);
             e1 = s;
         }
     }
-    if (lane == 0) a.carry[kNaSlots * k + 2] = __int_as_float(giant);
+    if (lane == 0) words.put(kNaSlots * k + 2, __int_as_float(giant));
 
     // ---- the other rows, tile by tile ----
     float open = 0.f;   // partial sum of row r, begun in an earlier tile
@@ -324,44 +354,59 @@ __device__ __forceinline__ void range_product(const NaArgs& a, int k, int lane, 
 }
 
 // The giant rows that begin in ranges [first, first + 32): their pieces in
-// range order (lane-strided, then a fixed tree).
-__device__ __forceinline__ void finish_giants(const NaArgs& a, int first, int lane) {
+// range order (lane-strided, then a fixed tree).  A range's row number counts
+// only if that row begins there and is a giant one in this call's row_ptr.
+template <class Words>
+__device__ __forceinline__ void finish_giants(const NaArgs& a, const Words& words, int first, int lane) {
     const int k = first + lane;
-    const int mine = k < a.ranges ? __float_as_int(__ldcg(a.carry + kNaSlots * k + 2)) : -1;
-    unsigned todo = __ballot_sync(0xffffffffu, mine >= 0);
+    const int mine = k < a.ranges ? __float_as_int(words.get(kNaSlots * k + 2)) : -1;
+    unsigned todo = __ballot_sync(0xffffffffu, mine >= 0 && mine < a.m);
     while (todo) {
         const int src = __ffs(int(todo)) - 1;
         todo &= todo - 1;
         const int row = __shfl_sync(0xffffffffu, mine, src);
         const int from = first + src;
-        const int end = min(max(__ldg(a.row_ptr + row + 1), 1), a.nnz);
+        const int s = __ldg(a.row_ptr + row), end = min(__ldg(a.row_ptr + row + 1), a.nnz);
+        if (s < from * a.T || s >= min((from + 1) * a.T, a.nnz) || end - s <= 2 * a.T) continue;
         const int to = min((end - 1) / a.T, a.ranges - 1);
         float t = 0.f;
-        for (int j = from + 1 + lane; j <= to; j += 32) t += __ldcg(a.carry + kNaSlots * j);
+        for (int j = from + 1 + lane; j <= to; j += 32) t += words.get(kNaSlots * j);
         t = warp_total(t);
-        if (lane == 0) a.y[row] = __ldcg(a.carry + kNaSlots * from + 1) + t;
+        if (lane == 0) a.y[row] = words.get(kNaSlots * from + 1) + t;
     }
 }
 
-template <bool kVec, bool kCluster>
+template <bool kVec>
 __global__ void __launch_bounds__(kNaWarps * 32, 6) noalloc_spmv_kernel(const NaArgs a) {
     __shared__ __align__(16) float products[kNaWarps][kNaTile];
     grid_dep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x * kNaWarps + warp;
-    if (k < a.ranges) range_product<kVec>(a, k, lane, products[warp]);
-    if constexpr (kCluster) {
-        // the whole product is this cluster: its pieces are visible after the barrier
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (32 * k < a.ranges) finish_giants(a, 32 * k, lane);
-    }
+    if (k < a.ranges) range_product<kVec>(a, GlobalWords{a.carry}, k, lane, products[warp]);
 }
 
 __global__ void __launch_bounds__(256) noalloc_giants_kernel(const NaArgs a) {
     grid_dep_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (32 * warp < a.ranges) finish_giants(a, 32 * warp, threadIdx.x & 31);
+    if (32 * warp < a.ranges) finish_giants(a, GlobalWords{a.carry}, 32 * warp, threadIdx.x & 31);
 }
+
+// The whole product by one cluster.
+template <bool kVec>
+__global__ void __launch_bounds__(kNaWarps * 32, 6) noalloc_cluster_kernel(const NaArgs a) {
+    __shared__ __align__(16) float products[kNaWarps][kNaTile];
+    __shared__ float pieces[kNaSlots * kNaWarps * kNaClusterBlocks];
+    cluster_arrive_relaxed();   // awaited by every warp before it writes to the first block
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = blockIdx.x * kNaWarps + warp;
+    const ClusterWords words(pieces);
+    if (k < a.ranges) range_product<kVec>(a, words, k, lane, products[warp]);
+    else words.ready();
+    // the pieces are visible after the barrier, to the first block's first two warps
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (32 * k < a.ranges) finish_giants(a, words, 32 * k, lane);
+}
+static_assert(kNaClusterBlocks * kNaWarps <= 32 * kNaWarps, "the first block finishes the cluster's giant rows");
 
 template <bool kVec>
 void launch(const NaArgs& a, cudaStream_t stream) {
@@ -378,10 +423,10 @@ void launch(const NaArgs& a, cudaStream_t stream) {
         attr[0].val.clusterDim.x = unsigned(blocks);
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        PB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, noalloc_spmv_kernel<kVec, true>, a));
+        PB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, noalloc_cluster_kernel<kVec>, a));
         return;
     }
-    noalloc_spmv_kernel<kVec, false><<<blocks, kNaWarps * 32, 0, stream>>>(a);
+    noalloc_spmv_kernel<kVec><<<blocks, kNaWarps * 32, 0, stream>>>(a);
     PB_CUDA_CHECK(cudaGetLastError());
     // launched while the product drains; it waits for it before it reads the pieces
     cfg.gridDim = dim3(unsigned((a.ranges + 255) / 256));

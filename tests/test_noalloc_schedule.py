@@ -1,0 +1,121 @@
+"""CPU restatement of the allocation-free product's schedule (noalloc.cu) in
+NumPy: the 32-probe search of a range's rows, the rows a range sums by itself,
+the pieces of giant rows (more than two ranges' entries) and the row numbers
+the ranges leave for the pass that adds them.
+
+Entries are small integers, so the sums are exact.  Larger products share one
+scratch array; the last test lets another call's words appear in it and checks
+that a row number is used only where it names a giant row of this call that
+begins in that range, so nothing is read or written outside [0, m) and products
+without giant rows keep their results."""
+import numpy as np
+import pytest
+
+TILE = 256
+
+
+def first_row(rp, m, target):
+    """First r in [0, m] with rp[r] >= target, by 32 probes a step."""
+    lo, width, steps = 0, m, 0
+    while width > 0:
+        stride = (width >> 5) + 1
+        probes = [rp[lo + q * stride] if q * stride < width else 2 ** 31 - 1 for q in range(32)]
+        hit = [q for q in range(32) if probes[q] >= target]
+        j = hit[0] if hit else 32
+        end = min(j * stride, width)
+        begin = (j - 1) * stride + 1 if j > 0 else 0
+        lo, width, steps = lo + begin, end - begin, steps + 1
+    assert steps <= 8
+    return lo
+
+
+def ranges(rp, e, T):
+    """(y, words): the rows that ranges write, and per range its piece of an
+    earlier giant row, its piece of one that begins here, and that row or -1."""
+    m, nnz = len(rp) - 1, int(rp[-1])
+    count = -(-nnz // T)
+    y, words = {}, np.zeros((count, 3), np.int64)
+    for k in range(count):
+        last = k == count - 1
+        lo, hi = k * T, nnz if last else (k + 1) * T
+        r, r1 = first_row(rp, m, lo), m if last else first_row(rp, m, hi)
+        assert r == np.searchsorted(rp[:m + 1], lo) or rp[r] >= lo
+        words[k, 2] = -1
+        if r > 0:
+            s, t = rp[r - 1], rp[r]
+            if t > lo and t - s > 2 * T:
+                words[k, 0] = e[lo:min(t, hi)].sum()
+        if r1 > r and rp[r1] - rp[r1 - 1] > 2 * T:
+            r1 -= 1
+            words[k, 1], words[k, 2] = e[rp[r1]:min(rp[r1 + 1], hi)].sum(), r1
+        for i in range(r, r1):
+            assert i not in y
+            y[i] = int(e[rp[i]:rp[i + 1]].sum())
+    return y, words
+
+
+def finish(rp, T, words, y):
+    """finish_giants: adds the pieces of the giant rows."""
+    m, nnz = len(rp) - 1, int(rp[-1])
+    for k, row in enumerate(words[:, 2]):
+        if not 0 <= row < m:
+            continue
+        s, end = rp[row], min(rp[row + 1], nnz)
+        if s < k * T or s >= min((k + 1) * T, nnz) or end - s <= 2 * T:
+            continue
+        to = min((end - 1) // T, len(words) - 1)
+        y[int(row)] = int(words[k, 1] + words[k + 1:to + 1, 0].sum())
+
+
+def operand(name, rng):
+    lens = {
+        "short": rng.integers(0, 9, 700),
+        "at_the_limit": np.array([2 * TILE, 2 * TILE + 1, 0, 1, TILE, 2 * TILE - 1, 3 * TILE, 5]),
+        "giants": np.where(np.arange(400) % 57 == 3, rng.integers(600, 3000, 400), rng.integers(0, 7, 400)),
+        "one_giant": np.array([0, 0, 9000, 0]),
+        "empty_ends": np.concatenate([np.zeros(700, int), rng.integers(0, 40, 60), np.zeros(900, int)]),
+        "giant_last": np.concatenate([rng.integers(0, 5, 90), [1300]]),
+    }[name]
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    return rp, rng.integers(-9, 10, rp[-1])
+
+
+NAMES = ["short", "at_the_limit", "giants", "one_giant", "empty_ends", "giant_last"]
+
+
+def sums(rp, e):
+    return [int(e[a:b].sum()) for a, b in zip(rp[:-1], rp[1:])]
+
+
+@pytest.mark.parametrize("tiles", [1, 3])
+@pytest.mark.parametrize("name", NAMES)
+def test_every_row_once(name, tiles):
+    rp, e = operand(name, np.random.default_rng(5))
+    y, words = ranges(rp, e, tiles * TILE)
+    giants = {int(r) for r in words[:, 2] if r >= 0}
+    assert not giants & set(y)
+    finish(rp, tiles * TILE, words, y)
+    assert [y[i] for i in range(len(rp) - 1)] == sums(rp, e)
+
+
+@pytest.mark.parametrize("other", NAMES)
+@pytest.mark.parametrize("name", NAMES)
+def test_another_calls_words_are_not_taken(name, other):
+    rng = np.random.default_rng(7)
+    rp, e = operand(name, rng)
+    rp2, e2 = operand(other, rng)
+    rp2 = np.concatenate([np.zeros(10_000, int), rp2])     # row numbers beyond the first call's m
+    y, words = ranges(rp, e, TILE)
+    foreign = ranges(rp2, e2, TILE)[1]
+    want = sums(rp, e)
+    giants = {i for i in range(len(rp) - 1) if rp[i + 1] - rp[i] > 2 * TILE}
+    for mixed in range(8):
+        w, out = words.copy(), dict(y)
+        n = min(len(w), len(foreign))
+        take = rng.random((n, 3)) < (1.0 if mixed == 0 else 0.5)
+        w[:n][take] = foreign[:n][take]
+        if mixed == 7:
+            w[:, 2] = rng.integers(-2 ** 31, 2 ** 31, len(w))
+        finish(rp, TILE, w, out)
+        assert set(out) <= set(range(len(rp) - 1))
+        assert all(out[i] == want[i] for i in out if i not in giants)
