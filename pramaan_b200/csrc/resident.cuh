@@ -50,7 +50,11 @@
 //
 // Waits are bounded (kWaitLimitNs): a block that gives up sets the status word
 // and leaves the loop, the blocks that wait for it follow, and all meet at the
-// last cluster barrier.
+// last cluster barrier.  A block that finished every iteration has waited for
+// every store sent to it.  One that gave up has not, and neither the barrier
+// nor its release covers them (st.async completes on the receiver's mbarrier
+// alone): past the barrier, when nobody sends any more, it stays for
+// kResDrainNs, far longer than a store is under way, before it retires.
 #pragma once
 
 #include <vector>
@@ -69,6 +73,9 @@ constexpr int kResWeights = 128;       // iterations whose weights are computed 
 constexpr int kResLongRow = 16;
 constexpr int kResFlat = 0, kResTiled = 1;
 constexpr uint16_t kResNoSlot = 0xffff;
+// How long a block that gave up outlives the last barrier (a remote store takes
+// about a microsecond).
+constexpr unsigned long long kResDrainNs = 10000000ull;   // 10 ms
 // Entries a long row takes: 2 modulo 16, so that the 8 rows a warp sums at a
 // time begin in different banks (rows of 48 back to back all began in the same
 // one: a block with 130 of them took 4,300 cycles for its half, 3,200 now).
@@ -688,7 +695,11 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResView 
         }
         for (int i = kResCached * kResThreads + tid; i < R; i += kResThreads) algo.y[me.r0 + i] = sy[i];
     }
-    cluster_barrier();   // no block leaves while another may still store into it
+    cluster_barrier();   // past it nobody stores into another block
+    if (!ok) {           // what was sent to a block that gave up may not have landed
+        const unsigned long long t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < kResDrainNs) __nanosleep(1000);
+    }
 }
 
 // The reference iteration: rows first (y from A x̄), then columns (x, x̄ from A^T y).
