@@ -100,7 +100,7 @@ public:
     bool has_lo = false;
     bool packed = false;
     bool align_rows = false;       // pack() starts a row that fits one tile in one tile (see align_rows_max)
-    bool aligned = false;          // pack() did so; the tile kernel takes the empty rows as well
+    bool aligned = false;          // pack() did so; the tile kernel takes a few empty rows as well
     bool keep_flat = false;        // pack() keeps the flat col / val (FP32) arrays
                                    // for kernels that read the plain CSR
     DevBuf<int> rp_c;              // non-empty rows' first entries, then nnz and nnz_pad (until pack())
@@ -115,7 +115,7 @@ public:
         CsrView v;
         v.rows = rows; v.cols = cols; v.nnz = nnz; v.nnz_pad = nnz_pad; v.num_tiles = num_tiles;
         v.rows_c = rows_c; v.num_cross = num_cross;
-        (aligned ? v.tile_empty : v.num_empty) = num_empty;
+        (aligned && num_empty <= tile_empty_max() ? v.tile_empty : v.num_empty) = num_empty;
         v.blocks_per_sm = tuned_blocks_per_sm;
         if (!packed && num_tiles > 0) throw std::logic_error("CsrDevice::view before pack()");
         v.rec = rec.get();
@@ -146,6 +146,16 @@ public:
     // row-aligned: uniform 0.4 M non-zeros 17.1 | 10.8, uniform 4 M 49.0 | 43.8,
     // banded 1 M 12.2 | 8.4, banded 26 M 101.2 | 92.9.
     static constexpr double align_rows_max = 0.08;
+    // Row-aligned tiles: the tile kernel does the empty rows while its warps (one
+    // per tile, about 2,048 at a time) take each lane no more than this many of
+    // them, one dependent pass after the other at its end.  More go to the fixup,
+    // whose launch has a thread for each.  us per reference iteration, empty
+    // columns in the tile kernel | fixup: 196 tiles, 5,000 (1 pass) 16.5 | 16.2,
+    // 20,000 (3.2) 18.4 | 16.3, 100,000 (16) 24.7 | 19.8, 1,000,000 (160) about 100 |
+    // 20; 2,000 tiles, 100,000 (1.5) 22.7 | 27.1, 200,000 (3) 22.9 | 24.9, 400,000 (6)
+    // 26.0 | 25.0; 8,000 tiles, 200,000 (3) 48.5 | 49.9, 800,000 (12) 56.3 | 55.9.
+    static constexpr int tile_empty_passes = 3;
+    int tile_empty_max() const { return tile_empty_passes * 32 * (num_tiles < 2048 ? num_tiles : 2048); }
     // Interleaves col / val / flags / meta into tile records and frees them
     // (entries whose target has a hot slot get ~slot).
     void pack(cudaStream_t st);

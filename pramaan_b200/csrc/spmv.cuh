@@ -79,9 +79,10 @@
 //
 // Completion (spmv_fixup_kernel, launched right after on the same stream)
 //   For every crossing row the fixup adds its pieces in tile order and runs
-//   the epilogue; it also gives every empty row the value 0 (with row-aligned
-//   tiles the tile kernel does).  All sums have a fixed order, so results are bit-identical between runs, and no thread
-//   ever waits on another block.
+//   the epilogue; it also gives every empty row the value 0 (a few of them the
+//   tile kernel does when the tiles are row-aligned).  All sums have a fixed
+//   order, so results are bit-identical between runs, and no thread ever waits
+//   on another block.
 #pragma once
 
 #include "common.cuh"
