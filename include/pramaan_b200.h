@@ -482,6 +482,13 @@ PRAMAAN_API int pramaan_session_panel_info(pramaan_pdhg_session* s, int32_t* pan
                                            int64_t* long_nnz, int32_t* min_len, int32_t* hot_rows,
                                            int64_t* hot_nnz);
 
+/* How the session's iterations run: the blocks of the thread-block cluster
+ * that keeps the LP in its shared memory (0: the products over tiles), and
+ * whether the tiles of the dual and the primal product hold whole rows.  Any
+ * pointer may be NULL. */
+PRAMAAN_API int pramaan_session_path_info(pramaan_pdhg_session* s, int32_t* cluster_blocks,
+                                          int32_t* aligned_dual, int32_t* aligned_primal);
+
 #ifdef __cplusplus
 }
 #endif

@@ -422,6 +422,16 @@ int pramaan_session_panel_info(pramaan_pdhg_session* s, int32_t* panels, int32_t
     });
 }
 
+int pramaan_session_path_info(pramaan_pdhg_session* s, int32_t* cluster_blocks, int32_t* aligned_dual,
+                              int32_t* aligned_primal) {
+    return guarded([&] {
+        if (!s) throw InvalidArgument("session is NULL");
+        if (cluster_blocks) *cluster_blocks = s->eng->cluster_blocks();
+        if (aligned_dual) *aligned_dual = s->eng->aligned_dual();
+        if (aligned_primal) *aligned_primal = s->eng->aligned_primal();
+    });
+}
+
 int pramaan_measure_gather_rate(const float* d_x, int32_t n, int32_t cached, int32_t reps,
                                 double* gathers_per_s) {
     return guarded([&] {

@@ -209,18 +209,19 @@ PdhgEngine::PdhgEngine(const pramaan_lp& lp, const pramaan_pdhg_options& opt) : 
         build_panel_split(A_, panel_, opt.panel_split, dev_, st_);
         build_panel_hot(A_, AT_, panel_, panel_t_, opt.gather_cache, dev_, st_);
     }
-    // Small LPs: the iterations run on one cluster, from the flat operands.
-    const int cluster = ResidentPlan::sizes_for({make_int4(m_, n_, lp.nnz, 0)}, device_sm_count(dev_))[0];
-    const bool small = !adaptive_ && !panel_.active && m_ > 0 && n_ > 0 && lp.nnz > 0 && cluster != 0 &&
-                       !opt.profile_kernels;
-    A_.keep_flat = AT_.keep_flat = small;
-    A_.align_rows = AT_.align_rows = !adaptive_ && !small;
+    // Small LPs: the iterations run on one cluster, from the flat operands.  Only
+    // the layout itself tells whether the LP fits, so the plan comes before the
+    // tiles: an LP that it refuses keeps no flat copy and gets row-aligned tiles.
+    if (!adaptive_ && !panel_.active && m_ > 0 && n_ > 0 && lp.nnz > 0 && !opt.profile_kernels) {
+        const int cluster = ResidentPlan::sizes_for({make_int4(m_, n_, lp.nnz, 0)}, device_sm_count(dev_))[0];
+        if (cluster != 0) resident_.build(A_, AT_, {make_int4(0, m_, 0, n_)}, cluster, st_);
+        resident_.prepare<ResReference>();
+        if (!resident_.ok()) resident_ = ResidentPlan{};
+    }
+    A_.keep_flat = AT_.keep_flat = resident_.ok();
+    A_.align_rows = AT_.align_rows = !adaptive_ && !resident_.ok();
     A_.pack(st_);
     AT_.pack(st_);
-    if (small) {
-        resident_.build(A_, AT_, {make_int4(0, m_, 0, n_)}, cluster, st_);
-        resident_.prepare<ResReference>();
-    }
     // the iteration's vectors: sigma, bounds, y (rows); tau, c, bounds, x, x̄ (columns), plus the gathers
     mark_l2_resident(A_, AT_, 20.0 * m_ + 28.0 * n_, dev_);
     // Occupancy queries / smem attributes before any graph capture.

@@ -72,6 +72,11 @@ public:
         *hot_rows = panel_t_.active ? panel_t_.hot_rows : 0;
         *hot_nnz = panel_t_.active ? panel_t_.hot_nnz : 0;
     }
+    // Blocks of the cluster that runs the iterations (0: the products over
+    // tiles), and whether a product's tiles hold whole rows.
+    int cluster_blocks() const { return resident_.ok() ? resident_.cluster_size() : 0; }
+    int aligned_dual() const { return panel_.active ? panel_.S.aligned : A_.aligned; }
+    int aligned_primal() const { return panel_t_.active ? panel_t_.rest.aligned : AT_.aligned; }
     int blocks_primal() const { return panel_t_.active ? panel_t_.rest.tuned_blocks_per_sm : AT_.tuned_blocks_per_sm; }
     void synchronize();
 

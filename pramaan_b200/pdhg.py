@@ -413,6 +413,14 @@ class Session:
         return {"panels": p.value, "long_rows": lr.value, "long_nnz": nz.value, "min_len": ml.value,
                 "primal_hot_rows": hr.value, "primal_hot_nnz": hz.value}
 
+    def path_info(self) -> dict:
+        """How the iterations run: the blocks of the cluster that keeps the LP
+        in its shared memory (0: the products over tiles), and whether the
+        tiles of A and of A^T hold whole rows."""
+        v = [C.c_int32() for _ in range(3)]
+        L.check(L.lib().pramaan_session_path_info(self._h, *(C.byref(q) for q in v)))
+        return {"cluster_blocks": v[0].value, "aligned": (bool(v[1].value), bool(v[2].value))}
+
     def gather_slots(self) -> tuple[int, int]:
         """Hot gather slots of A and A^T."""
         g = self.gather_info()
