@@ -439,7 +439,11 @@ void PdhgEngine::build_graph(int k) {
 
 void PdhgEngine::iterate(int k) {
     if (k <= 0) return;
-    if (resident_.ok()) {
+    // A launch on the cluster begins with loading the LP, which a few iterations
+    // over tiles undercut.  us for a call of k iterations and a wait, tiles |
+    // cluster: 12 K non-zeros k = 1 24 | 33, k = 2 32 | 33; 36 K k = 2 32 | 40, k = 4
+    // 49 | 45; 60 K k = 3 40 | 50, k = 6 62 | 61; 100 K k = 5 68 | 85, k = 8 98 | 98.
+    if (resident_.ok() && k >= 2 + A_.nnz / 15000) {
         const ResReference algo{x_.get(),  xbar_.get(), y_.get(),  tau_.get(), c_.get(), lx_.get(),
                                 ux_.get(), sigma_.get(), lr_.get(), ur_.get(), nullptr};
         resident_.launch(A_, AT_, algo, k, status_.get(), st_);

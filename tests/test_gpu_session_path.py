@@ -51,6 +51,22 @@ def test_tiles_hold_whole_rows_unless_they_would_be_too_many(name, aligned):
     assert _path(md, profile_kernels=True)["aligned"][0] is aligned
 
 
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("shape", [(100, 200, 4), (1000, 3000, 4), (5000, 15000, 4)])
+def test_calls_of_few_and_of_many_iterations_follow_each_other(shape, graph):
+    """Calls of a few iterations run over tiles (loading the LP into a cluster
+    would take longer), longer ones on the cluster, on the same iterates."""
+    md = random_sparse_lp(*shape, seed=4)
+    with Session(md, PdhgOptions(use_graph=graph)) as s:
+        assert s.path_info()["cluster_blocks"] > 0
+        for k in (1, 1, 9, 2, 5, 1, 20, 3):
+            s.iterate(k)
+        x, y = s.iterates()
+    rx, ry, _ = oracle.trajectory(md, 42)
+    np.testing.assert_allclose(x, rx, rtol=1e-4, atol=1e-4)
+    np.testing.assert_allclose(y, ry, rtol=1e-4, atol=1e-4 * (1 + np.abs(ry).max()))
+
+
 def test_graph_replay_and_direct_launches_agree_bitwise():
     """The reference iteration over tiles: an LP that no cluster's shared memory
     holds, with rows from one entry to 1,000 (crossing rows), as a CUDA graph and
