@@ -48,8 +48,17 @@ __global__ void cold_x_kernel(const double* __restrict__ lo, const double* __res
     }
 }
 
-__global__ void minimise_kernel(const double* __restrict__ c, int n, bool maximise, double* __restrict__ out) {
-    CERT_STRIDE(j, n) out[j] = maximise ? -c[j] : c[j];
+// out[j] = c[j], negated in the LPs that maximise; lps[k] = {first column, maximises}.
+__global__ void minimise_kernel(const double* __restrict__ c, int n, const int2* __restrict__ lps, int count,
+                                double* __restrict__ out) {
+    CERT_STRIDE(j, n) {
+        int lo = 0, hi = count - 1;   // the last LP that begins at or before j
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (lps[mid].x <= j) lo = mid; else hi = mid - 1;
+        }
+        out[j] = lps[lo].y ? -c[j] : c[j];
+    }
 }
 
 // rows: slots 0-3 sums (rp2, b2, dobj, rd2), slot 7 max row violation
@@ -190,11 +199,6 @@ CertificateBatch::CertificateBatch(const pramaan_lp* lps, int count, int device)
     PB_CUDA_CHECK(cudaMemsetAsync(status_.get(), 0, 4, st_));
     const size_t Mz = size_t(m_), Nz = size_t(n_);
     rlo_.alloc(Mz); rhi_.alloc(Mz); vlo_.alloc(Nz); vhi_.alloc(Nz); cmin_.alloc(Nz); cmod_.alloc(Nz);
-    // Straight from the caller's arrays: packing them on the host first took more
-    // than half of a call (32 planning LPs and three points: 13.1 ms, 8.3 ms now).
-    auto to = [&](DevBuf<double>& d, int at, const double* h, int len) {
-        if (len > 0) PB_CUDA_CHECK(cudaMemcpyAsync(d.get() + at, h, size_t(len) * 8, cudaMemcpyHostToDevice, st_));
-    };
     std::vector<CsrPart> parts;
     for (int k = 0; k < count; ++k) {
         const pramaan_lp& lp = lps[k];
@@ -204,17 +208,32 @@ CertificateBatch::CertificateBatch(const pramaan_lp* lps, int count, int device)
         parts.push_back(CsrPart{lp.row_ptr, lp.col_idx, lp.values, lp.num_rows, lp.num_cols, lp.nnz});
     }
     csr_upload_f64_parts(A_, m_, n_, nnz_, parts, st_);
+    // Straight from the caller's arrays where they are large: packing them all on
+    // the host took more than half of a call (32 planning LPs and three points:
+    // 13.1 ms, 8.3 ms now).
+    PackedUpload<double> rlo(rlo_.get(), st_), rhi(rhi_.get(), st_), cost(cmod_.get(), st_), vlo(vlo_.get(), st_),
+        vhi(vhi_.get(), st_);
+    std::vector<int2> sense;
+    for (int k = 0; k < count; ++k) {
+        const size_t R = size_t(lps[k].num_rows), C = size_t(lps[k].num_cols);
+        for (auto* u : {&rlo, &rhi}) u->expect(R);
+        for (auto* u : {&cost, &vlo, &vhi}) u->expect(C);
+        sense.push_back(make_int2(c0_[size_t(k)], lps[k].obj_sense == PRAMAAN_MAXIMIZE));
+    }
     for (int k = 0; k < count; ++k) {
         const pramaan_lp& lp = lps[k];
-        const int R = r0_[size_t(k)], C = c0_[size_t(k)];
-        to(rlo_, R, lp.row_lower, lp.num_rows);
-        to(rhi_, R, lp.row_upper, lp.num_rows);
-        to(cmod_, C, lp.obj_coeffs, lp.num_cols);
-        to(vlo_, C, lp.var_lower, lp.num_cols);
-        to(vhi_, C, lp.var_upper, lp.num_cols);
-        if (lp.num_cols > 0)
-            minimise_kernel<<<grid(lp.num_cols), kThreads, 0, st_>>>(cmod_.get() + C, lp.num_cols,
-                                                                    lp.obj_sense == PRAMAAN_MAXIMIZE, cmin_.get() + C);
+        const size_t R = size_t(lp.num_rows), C = size_t(lp.num_cols);
+        rlo.add(lp.row_lower, R);
+        rhi.add(lp.row_upper, R);
+        cost.add(lp.obj_coeffs, C);
+        vlo.add(lp.var_lower, C);
+        vhi.add(lp.var_upper, C);
+    }
+    for (auto* u : {&rlo, &rhi, &cost, &vlo, &vhi}) u->flush();
+    DevBuf<int2> d_sense(sense.size());
+    if (n_ > 0) {
+        PB_CUDA_CHECK(cudaMemcpyAsync(d_sense.get(), sense.data(), sense.size() * sizeof(int2), cudaMemcpyHostToDevice, st_));
+        minimise_kernel<<<grid(n_), kThreads, 0, st_>>>(cmod_.get(), n_, d_sense.get(), count, cmin_.get());
     }
     PB_CUDA_CHECK(cudaGetLastError());
     csr_transpose(A_, AT_, st_);
@@ -255,16 +274,25 @@ void CertificateBatch::evaluate(const pramaan_warm_start* points, pramaan_certif
     if (K == 0) return;
     // the point in the packed layout (x NULL: the cold start; y NULL: 0)
     std::vector<char> cold(size_t(K), 0);
+    PackedUpload<double> ux(x_.get(), st_), uy(y_.get(), st_);
+    bool zero_y = false;
+    for (int k = 0; k < K; ++k) {
+        if (points[k].x) ux.expect(size_t(c0_[size_t(k) + 1] - c0_[size_t(k)]));
+        if (points[k].y) uy.expect(size_t(r0_[size_t(k) + 1] - r0_[size_t(k)]));
+        else zero_y = true;
+    }
+    if (zero_y && m_ > 0) PB_CUDA_CHECK(cudaMemsetAsync(y_.get(), 0, size_t(m_) * 8, st_));
     for (int k = 0; k < K; ++k) {
         const pramaan_warm_start& p = points[k];
-        const int C = c0_[size_t(k)], R = r0_[size_t(k)];
-        const size_t nk = size_t(c0_[size_t(k) + 1] - C), mk = size_t(r0_[size_t(k) + 1] - R);
+        const size_t nk = size_t(c0_[size_t(k) + 1] - c0_[size_t(k)]), mk = size_t(r0_[size_t(k) + 1] - r0_[size_t(k)]);
         cold[size_t(k)] = p.x ? 0 : 1;
-        if (p.x && nk > 0) PB_CUDA_CHECK(cudaMemcpyAsync(x_.get() + C, p.x, nk * 8, cudaMemcpyHostToDevice, st_));
-        if (mk == 0) continue;
-        if (p.y) PB_CUDA_CHECK(cudaMemcpyAsync(y_.get() + R, p.y, mk * 8, cudaMemcpyHostToDevice, st_));
-        else PB_CUDA_CHECK(cudaMemsetAsync(y_.get() + R, 0, mk * 8, st_));
+        if (p.x) ux.add(p.x, nk);
+        else ux.skip(nk);
+        if (p.y) uy.add(p.y, mk);
+        else uy.skip(mk);
     }
+    ux.flush();
+    uy.flush();
     // cold-start LPs: x0 = clamp(0, l, u) over their columns
     for (int k = 0; k < K; ++k) {
         if (!cold[size_t(k)]) continue;

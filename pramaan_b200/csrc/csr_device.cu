@@ -776,19 +776,26 @@ void csr_upload_f64_parts(CsrDevice& A, int rows, int cols, int nnz, const std::
     DevBuf<int4> at{parts.size()};
     PB_CUDA_CHECK(cudaMemsetAsync(flag.get(), 0, 4, st));
     std::vector<int4> first;
+    PackedUpload<int> up_rows(A.row_ptr.get(), st), up_col(A.col.get(), st);
+    PackedUpload<double> up_val(v64.get(), st);
+    for (const CsrPart& p : parts) {
+        up_rows.expect(size_t(p.rows));
+        up_col.expect(size_t(p.nnz));
+        up_val.expect(size_t(p.nnz));
+    }
     size_t r0 = 0, e0 = 0, c0 = 0;
     for (const CsrPart& p : parts) {
         first.push_back(make_int4(int(r0), int(e0), int(c0), p.cols));
-        if (p.rows > 0)
-            PB_CUDA_CHECK(cudaMemcpyAsync(A.row_ptr.get() + r0, p.row_ptr, size_t(p.rows) * 4, cudaMemcpyHostToDevice, st));
-        if (p.nnz > 0) {
-            PB_CUDA_CHECK(cudaMemcpyAsync(A.col.get() + e0, p.col, size_t(p.nnz) * 4, cudaMemcpyHostToDevice, st));
-            PB_CUDA_CHECK(cudaMemcpyAsync(v64.get() + e0, p.val, size_t(p.nnz) * 8, cudaMemcpyHostToDevice, st));
-        }
+        up_rows.add(p.row_ptr, size_t(p.rows));
+        up_col.add(p.col, size_t(p.nnz));
+        up_val.add(p.val, size_t(p.nnz));
         r0 += size_t(p.rows);
         e0 += size_t(p.nnz);
         c0 += size_t(p.cols);
     }
+    up_rows.flush();
+    up_col.flush();
+    up_val.flush();
     PB_CUDA_CHECK(cudaMemcpyAsync(at.get(), first.data(), first.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
     shift_parts_kernel<<<grid_1d((long long)rows + nnz + 1), kThreads, 0, st>>>(A.row_ptr.get(), A.col.get(), at.get(),
                                                                               int(parts.size()), rows, nnz, flag.get());
