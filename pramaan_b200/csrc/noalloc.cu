@@ -119,7 +119,7 @@ __device__ __forceinline__ void first_rows(const int* __restrict__ rp, int m, in
             const unsigned yes = __ballot_sync(0xffffffffu, probe[q] >= target[q]);
             if (width[q] == 0) continue;
             const int j = yes ? __ffs(int(yes)) - 1 : 32;   // first probe at or above the target
-            const int end = min(j * stride[q], width[q]);
+            const int end = int(min(unsigned(j) * unsigned(stride[q]), unsigned(width[q])));   // 32 strides: up to 2^31
             const int begin = j > 0 ? (j - 1) * stride[q] + 1 : 0;
             lo[q] += begin;
             width[q] = end - begin;
@@ -313,23 +313,24 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
     for (int base = e0 & ~3; base < e1; base += kNaTile) {
         const int lim = base + kNaTile;
         // the row pointers of the next 32 rows travel with the tile's entries
-        int s = r + lane <= r1 ? rp(r + lane) : INT_MAX;
-        int s_next = r + 32 <= r1 ? rp(r + 32) : INT_MAX;
+        // (r1 - r, not r + 32: row numbers may go up to INT_MAX)
+        int s = lane <= r1 - r ? rp(r + lane) : INT_MAX;
+        int s_next = 32 <= r1 - r ? rp(r + 32) : INT_MAX;
         if (base >= e0 && lim <= e1) tile_products<kVec, false>(a, base, e0, e1, last_col, lane, p);
         else tile_products<kVec, true>(a, base, e0, e1, last_col, lane, p);
         __syncwarp();
         while (true) {
             int e = __shfl_down_sync(0xffffffffu, s, 1);
             if (lane == 31) e = s_next;
-            const bool started = r + lane < r1 && s < lim;
+            const bool started = lane < r1 - r && s < lim;
             const bool done = started && e <= lim;
             const unsigned started_m = __ballot_sync(0xffffffffu, started);
             const int nd = __popc(__ballot_sync(0xffffffffu, done));
             // the next rows' pointers, before the sums of these
             int s2 = INT_MAX, s2_next = INT_MAX;
             if (nd == 32) {
-                s2 = r + 32 + lane <= r1 ? rp(r + 32 + lane) : INT_MAX;
-                s2_next = r + 64 <= r1 ? rp(r + 64) : INT_MAX;
+                s2 = 32 + lane <= r1 - r ? rp(r + 32 + lane) : INT_MAX;
+                s2_next = 64 <= r1 - r ? rp(r + 64) : INT_MAX;
             }
             const int from = started ? max(s, base) - base : 0;
             const int to = started ? min(e, lim) - base : 0;
@@ -350,7 +351,8 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
         }
         __syncwarp();   // p is free for the next tile
     }
-    for (int i = r + lane; i < r1; i += 32) a.y[i] = 0.f;   // empty rows after the last entry
+    // empty rows after the last entry
+    for (unsigned i = unsigned(r) + unsigned(lane); i < unsigned(r1); i += 32) a.y[i] = 0.f;
 }
 
 // The giant rows that begin in ranges [first, first + 32): their pieces in

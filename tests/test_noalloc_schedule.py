@@ -15,7 +15,8 @@ TILE = 256
 
 
 def first_row(rp, m, target):
-    """First r in [0, m] with rp[r] >= target, by 32 probes a step."""
+    """First r in [0, m] with rp[r] >= target, by 32 probes a step; the kernel's
+    products are 32 bits wide, the end of a step unsigned."""
     lo, width, steps = 0, m, 0
     while width > 0:
         stride = (width >> 5) + 1
@@ -24,6 +25,7 @@ def first_row(rp, m, target):
         j = hit[0] if hit else 32
         end = min(j * stride, width)
         begin = (j - 1) * stride + 1 if j > 0 else 0
+        assert 31 * stride < 2 ** 31 and j * stride < 2 ** 32 and begin < 2 ** 31
         lo, width, steps = lo + begin, end - begin, steps + 1
     assert steps <= 8
     return lo
@@ -119,3 +121,23 @@ def test_another_calls_words_are_not_taken(name, other):
         finish(rp, TILE, w, out)
         assert set(out) <= set(range(len(rp) - 1))
         assert all(out[i] == want[i] for i in out if i not in giants)
+
+
+class _Steps:
+    """A row_ptr of m + 1 entries that is 0 up to row `at` and 7 from there on."""
+
+    def __init__(self, at):
+        self.at = at
+
+    def __getitem__(self, i):
+        return 7 if i >= self.at else 0
+
+
+@pytest.mark.parametrize("m", [2 ** 31 - 1, 2 ** 31 - 2, 2 ** 31 - 32, 2 ** 31 - 33, 2 ** 30 + 1])
+def test_search_over_the_most_rows(m):
+    """The 32nd stride of a search over 2^31 - 32 rows and more ends at 2^31,
+    which is no int."""
+    assert 32 * (((2 ** 31 - 32) >> 5) + 1) == 2 ** 31
+    for at in (0, 1, 31, 32, m // 2, m - 33, m - 1, m):
+        assert first_row(_Steps(at), m, 7) == at
+        assert first_row(_Steps(at), m, 0) == 0
