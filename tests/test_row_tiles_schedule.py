@@ -128,3 +128,15 @@ def test_crossing_rows_by_compacted_index_would_be_wrong():
     by_map = aligned_tiles(rp_c, row_map)[1]
     by_index = aligned_tiles(rp_c, np.arange(len(row_map)))[1]
     assert [c[0] for c in by_map] == [40] and [c[0] for c in by_index] == [38]
+
+
+@pytest.mark.parametrize("entries", [1, 5, 15, 16, 17, 100, 495, 496, 497, 511])
+def test_padding_repeats_a_column_of_its_own_load(entries):
+    """pad_source: a lane holds 16 consecutive entries and entry j of all lanes is
+    one load; padding repeats an entry of the same load, or the last entry where
+    the tile has none."""
+    for k in range(entries, 512):
+        q = k - ((k - entries) // 16 + 1) * 16
+        q = q if q >= 0 else entries - 1
+        assert 0 <= q < entries
+        assert q % 16 == k % 16 or entries < 16
