@@ -274,6 +274,26 @@ struct ClusterWords {
     __device__ __forceinline__ float get(int i) const { return own[i]; }
 };
 
+// Writes zeros to the empty rows at the front of [r, r1), whose row pointer is v
+// (so is that of the row before): found 32, then 1,024, 32,768, ... rows to a lane
+// and load.  Row by row the warp that owns a long run would read all its pointers
+// 32 at a time.  Returns the first row left; runs shorter than 32 are left too.
+template <class RowPtr>
+__device__ __forceinline__ int skip_empty(const NaArgs& a, const RowPtr& rp, int v, int r, int r1, int lane) {
+    int stride = 32;
+    while (stride <= r1 - r) {
+        const unsigned ahead = unsigned(stride) * unsigned(lane + 1);   // at most 2^30
+        const bool empty = ahead <= unsigned(r1 - r) && rp(r + int(ahead)) == v;
+        const int strides = __popc(__ballot_sync(0xffffffffu, empty));
+        const int end = r + stride * strides;
+        for (int i = r + lane; i < end; i += 32) a.y[i] = 0.f;
+        r = end;
+        if (strides < 32 && stride == 32) break;
+        stride = strides < 32 ? 32 : min(stride * 32, 1 << 25);
+    }
+    return r;
+}
+
 // One range by one warp.
 template <bool kVec, class Words>
 __device__ __forceinline__ void range_product(const NaArgs& a, const Words& words, int k, int lane, float* __restrict__ p) {
@@ -328,6 +348,14 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
             const int nd = __popc(__ballot_sync(0xffffffffu, done));
             // the next rows' pointers, before the sums of these
             int s2 = INT_MAX, s2_next = INT_MAX;
+            const int v = __shfl_sync(0xffffffffu, s, 0);
+            if (nd == 32 && s_next == v) {   // 32 empty rows: zeros, and on to the last row of the run
+                a.y[r + lane] = 0.f;
+                r = skip_empty(a, rp, v, r + 32, r1, lane);
+                s = lane <= r1 - r ? rp(r + lane) : INT_MAX;
+                s_next = 32 <= r1 - r ? rp(r + 32) : INT_MAX;
+                continue;
+            }
             if (nd == 32) {
                 s2 = 32 + lane <= r1 - r ? rp(r + 32 + lane) : INT_MAX;
                 s2_next = 64 <= r1 - r ? rp(r + 64) : INT_MAX;

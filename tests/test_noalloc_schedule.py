@@ -89,14 +89,15 @@ def sums(rp, e):
     return [int(e[a:b].sum()) for a, b in zip(rp[:-1], rp[1:])]
 
 
-@pytest.mark.parametrize("tiles", [1, 3])
+@pytest.mark.parametrize("tiles", [0.25, 0.5, 1, 3])
 @pytest.mark.parametrize("name", NAMES)
 def test_every_row_once(name, tiles):
     rp, e = operand(name, np.random.default_rng(5))
-    y, words = ranges(rp, e, tiles * TILE)
+    T = int(tiles * TILE)
+    y, words = ranges(rp, e, T)
     giants = {int(r) for r in words[:, 2] if r >= 0}
     assert not giants & set(y)
-    finish(rp, tiles * TILE, words, y)
+    finish(rp, T, words, y)
     assert [y[i] for i in range(len(rp) - 1)] == sums(rp, e)
 
 
@@ -141,3 +142,36 @@ def test_search_over_the_most_rows(m):
     for at in (0, 1, 31, 32, m // 2, m - 33, m - 1, m):
         assert first_row(_Steps(at), m, 7) == at
         assert first_row(_Steps(at), m, 0) == 0
+
+
+def skip_empty(rp, v, r, r1, cleared):
+    """skip_empty of the kernel: probes of 32 lanes at growing strides."""
+    stride = 32
+    while stride <= r1 - r:
+        empty = [stride * (q + 1) <= r1 - r and rp[r + stride * (q + 1)] == v for q in range(32)]
+        strides = sum(empty)
+        cleared.extend(range(r, r + stride * strides))
+        r += stride * strides
+        if strides < 32 and stride == 32:
+            break
+        stride = 32 if strides < 32 else min(stride * 32, 1 << 25)
+    return r
+
+
+@pytest.mark.parametrize("after", [0, 1, 40])
+@pytest.mark.parametrize("run", [0, 1, 31, 32, 33, 63, 64, 1023, 1024, 1025, 1056, 1088, 33_000, 33_900, 70_001])
+def test_runs_of_empty_rows(run, after):
+    """Clears the front of the run and nothing else, and leaves fewer than 32 of
+    its rows (or, near the end of the range, fewer than the stride it stood at)."""
+    v = 5
+    rp = np.concatenate([np.full(run + 1, v), v + 1 + np.arange(after)])
+    r1, cleared = len(rp) - 1, []
+    r = 0
+    for _ in range(8):                       # the kernel comes back after every 32 empty rows
+        r = skip_empty(rp, v, r, r1, cleared)
+        if r + 32 > r1 or rp[r + 32] != v:
+            break
+        cleared.extend(range(r, r + 32))
+        r += 32
+    assert cleared == list(range(r)) and r <= run
+    assert run - r < 64
