@@ -36,12 +36,13 @@
 // round trips.  Measured per call in a captured graph (before: tiles of 2,048
 // entries per block, serial searches by one thread, a completion kernel that
 // searched again):
-//   1,000 x 3,000, 12 K entries              5.3 us
-//   200,000 x 500,000, 4 M, uniform         25.7 us   (58.8 us of kernel time)
-//   500,000 x 1,250,000, 27 M, power law     136 us   (238 us of kernel time)
-//   the same size, 25.6 M, banded             61 us   (0.53 of the HBM copy rate)
+//   1,000 x 3,000, 12 K entries              4.9 us   (10.2 us)
+//   200,000 x 500,000, 4 M, uniform         24.8 us   (45.0 us)
+//   500,000 x 1,250,000, 27 M, power law     134 us   (228 us)
+//   the same size, 25.5 M, banded             54 us   (166 us; 0.59 of the HBM copy rate)
 // Tiles of 512 entries (64 registers, 32 warps per SM instead of 48) cost
-// 65 us on the banded and 18 against 16.5 us on a 1 M-entry product.
+// 65 us on the banded and 18 against 16.5 us on a 1 M-entry product, when the
+// shipped tiles took 61 us there.
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -249,28 +250,40 @@ __device__ __forceinline__ float row_sums(const float* __restrict__ p, int from,
     return sum;
 }
 
-__device__ __forceinline__ void cluster_arrive_relaxed() {
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // Where the ranges leave their words: the scratch array, or the shared memory
-// of the cluster's first block.
+// of the cluster's first block.  ready() comes before put(), by the whole warp.
 struct GlobalWords {
     float* at;
     __device__ __forceinline__ void ready() const {}
     __device__ __forceinline__ void put(int i, float v) const { at[i] = v; }
+    // range k's giant row, or -1 (what is there may be another call's)
+    __device__ __forceinline__ void mark(int k, int row, int lane) const {
+        if (lane == 0) at[kNaSlots * k + 2] = __int_as_float(row);
+    }
     __device__ __forceinline__ float get(int i) const { return __ldcg(at + i); }
 };
 struct ClusterWords {
-    float* own;       // this block's array (the first block's is the one in use)
-    uint32_t first;   // the first block's, as an address in the cluster
+    float* own;                // this block's array (the first block's is the one in use)
+    mutable bool waited = false;
+    // The first block's marks start as -1, so a range without a giant row stores nothing.
     __device__ explicit ClusterWords(float* shared) : own(shared) {
-        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(first) : "r"(smem_u32(shared)));
+        if (threadIdx.x < kNaWarps * kNaClusterBlocks) own[kNaSlots * threadIdx.x + 2] = __int_as_float(-1);
+        cluster_arrive();
     }
-    __device__ __forceinline__ void ready() const { cluster_wait(); }   // the first block runs
+    __device__ __forceinline__ void ready() const {   // the first block runs and its marks are set
+        if (!waited) cluster_wait();
+        waited = true;
+    }
     __device__ __forceinline__ void put(int i, float v) const {
+        uint32_t first;
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(first) : "r"(smem_u32(own)));
         asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(first + 4u * unsigned(i)), "f"(v) : "memory");
+    }
+    __device__ __forceinline__ void mark(int k, int row, int lane) const {
+        if (row >= 0 && lane == 0) put(kNaSlots * k + 2, __int_as_float(row));
     }
     __device__ __forceinline__ float get(int i) const { return own[i]; }
 };
@@ -309,11 +322,11 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
     int e1 = r1 > r ? rp(r1) : 0;
     // ---- pieces of giant rows ----
     const int kGiant = 2 * a.T;
-    words.ready();
     if (r > 0) {
         const int s = rp(r - 1), e = r1 > r ? e0 : rp(r);
         if (e > lo && e - s > kGiant) {
             const float t = piece_sum(a, lo, min(e, hi), last_col, lane);
+            words.ready();
             if (lane == 0) words.put(kNaSlots * k, t);
         }
     }
@@ -323,11 +336,12 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
         if (e1 - s > kGiant) {
             giant = --r1;
             const float t = piece_sum(a, s, min(e1, hi), last_col, lane);
+            words.ready();
             if (lane == 0) words.put(kNaSlots * k + 1, t);
             e1 = s;
         }
     }
-    if (lane == 0) words.put(kNaSlots * k + 2, __int_as_float(giant));
+    words.mark(k, giant, lane);
 
     // ---- the other rows, tile by tile ----
     float open = 0.f;   // partial sum of row r, begun in an earlier tile
@@ -441,14 +455,14 @@ template <bool kVec>
 __global__ void __launch_bounds__(kNaWarps * 32, 6) noalloc_cluster_kernel(const NaArgs a) {
     __shared__ __align__(16) float products[kNaWarps][kNaTile];
     __shared__ float pieces[kNaSlots * kNaWarps * kNaClusterBlocks];
-    cluster_arrive_relaxed();   // awaited by every warp before it writes to the first block
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x * kNaWarps + warp;
     const ClusterWords words(pieces);
     if (k < a.ranges) range_product<kVec>(a, words, k, lane, products[warp]);
-    else words.ready();
+    words.ready();
     // the pieces are visible after the barrier, to the first block's first two warps
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
     if (32 * k < a.ranges) finish_giants(a, words, 32 * k, lane);
 }
 static_assert(kNaClusterBlocks * kNaWarps <= 32 * kNaWarps, "the first block finishes the cluster's giant rows");
@@ -530,14 +544,24 @@ void spmv_noalloc(const int32_t* d_row_ptr, const int32_t* d_col_idx, const floa
         PB_CUDA_CHECK(cudaMemsetAsync(d_y, 0, size_t(m) * sizeof(float), stream));
         return;
     }
-    // Tiles per range: one, so that a small product spreads over the chip
-    // (1.07 M entries: 16.5 us with one, 25.9 with four), up to four from 4 Mi
-    // entries on, where the ranges fill it anyway and fewer searches pay (4 M
-    // entries: 27.8 us with one, 25.7 with four), more only where the scratch
-    // would not hold the ranges.
+    // Tiles per range: one per Mi entries, between one, so that a small product
+    // spreads over the chip, and four, where the ranges fill it anyway and fewer
+    // searches pay; more only where the scratch would not hold the ranges.  us with
+    // 1 | 2 | 3 | 4 tiles: 1 M entries uniform 12.1 | 11.2 | 13.5 | 12.0, power law 13.1 |
+    // 14.3 | 17.4 | 19.3; 2.2 M uniform 19.2 | 15.9 | 16.9 | 16.0, banded 12.7 | 9.8 | 9.6 |
+    // 9.7; 4 M uniform 27.9 | 26.6 | 24.7 | 25.6, banded 18.7 | 15.0 | 12.9 | 13.3; 8 M uniform
+    // 48.9 | 42.7 | 41.0 | 44.6.
     const int by_size = std::min(std::max(nnz >> 20, 1), 4);
     const int by_scratch = int((nnz + (long long)kNaTile * kNaMaxRanges - 1) / ((long long)kNaTile * kNaMaxRanges));
-    const int T = kNaTile * std::max(by_size, by_scratch);
+    // Products of up to 64 ranges (a cluster's warps) of a quarter or half a tile
+    // take such short ranges: their warps' work is mostly rows, 32 a step, and long
+    // rows are cut finer.  us with ranges of 256 | 64 entries (before: one block per
+    // 2,048 entries): 1,000 rows of one entry 6.4 | 4.2 (5.6), 50 rows of 40 4.5 | 3.8
+    // (4.7), 2 rows of 1,000 5.1 | 4.3 (4.3); of 128: 2,000 rows of 4 4.6 | 4.3 (10.6).
+    const int cluster_ranges = kNaWarps * kNaClusterBlocks;
+    const int T = nnz <= cluster_ranges * (kNaTile / 4)   ? kNaTile / 4
+                  : nnz <= cluster_ranges * (kNaTile / 2) ? kNaTile / 2
+                                                          : kNaTile * std::max(by_size, by_scratch);
     const NaArgs a{d_row_ptr, d_col_idx, d_values, d_x, d_y, carry, m, n, nnz, T, (nnz + T - 1) / T};
     const bool vec = ((reinterpret_cast<uintptr_t>(d_col_idx) | reinterpret_cast<uintptr_t>(d_values)) & 15) == 0;
     if (vec) launch<true>(a, stream);
