@@ -70,11 +70,10 @@ constexpr int kNaLocalSpan = 16384;                  // columns: a tile within t
 __device__ __align__(256) float g_noalloc_carry[131072];
 static_assert(kNaSlots * kNaMaxRanges <= 131072, "scratch words");
 
-// Per device ordinal: the array's device address and the SM count, looked up
+// Per device ordinal: the array's device address, looked up
 // once with that device current.  The address belongs to the runtime's primary
 // context of the device, the one every call of this entry point uses.
 std::atomic<float*> g_carry_addr[64];
-std::atomic<int> g_sm_count[64];
 std::mutex g_setup_mutex;
 
 struct NaArgs {
@@ -495,29 +494,22 @@ void launch(const NaArgs& a, cudaStream_t stream) {
     PB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, noalloc_giants_kernel, a));
 }
 
-// Device address of the scratch array for `dev` (and its SM count), looked up
+// Device address of the scratch array for `dev`, looked up
 // once per device with that device current and cached.  With lazy module
 // loading this first lookup is also where the module, and with it the array,
 // may be loaded onto the device.
-float* carry_address(int dev, int* sms) {
+float* carry_address(int dev) {
     if (dev < 0 || dev >= 64) throw InvalidArgument("device ordinal out of range");
     float* p = g_carry_addr[dev].load(std::memory_order_acquire);
-    if (p) {
-        *sms = g_sm_count[dev].load(std::memory_order_relaxed);
-        return p;
-    }
+    if (p) return p;
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     p = g_carry_addr[dev].load(std::memory_order_relaxed);
     if (!p) {
-        int count = 0;
-        PB_CUDA_CHECK(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
         void* addr = nullptr;
         PB_CUDA_CHECK(cudaGetSymbolAddress(&addr, g_noalloc_carry));
         p = static_cast<float*>(addr);
-        g_sm_count[dev].store(count, std::memory_order_relaxed);
         g_carry_addr[dev].store(p, std::memory_order_release);
     }
-    *sms = g_sm_count[dev].load(std::memory_order_relaxed);
     return p;
 }
 
@@ -538,8 +530,7 @@ void spmv_noalloc(const int32_t* d_row_ptr, const int32_t* d_col_idx, const floa
         throw InvalidArgument("col_idx, values and x must not be NULL (and n > 0) when nnz > 0");
     int dev = 0;
     PB_CUDA_CHECK(cudaGetDevice(&dev));
-    int sms = 0;
-    float* carry = carry_address(dev, &sms);
+    float* carry = carry_address(dev);
     if (nnz == 0) {
         PB_CUDA_CHECK(cudaMemsetAsync(d_y, 0, size_t(m) * sizeof(float), stream));
         return;
