@@ -299,7 +299,7 @@ __device__ __forceinline__ int skip_empty(const NaArgs& a, const RowPtr& rp, int
         const bool empty = ahead <= unsigned(r1 - r) && rp(r + int(ahead)) == v;
         const int strides = __popc(__ballot_sync(0xffffffffu, empty));
         const int end = r + stride * strides;
-        for (int i = r + lane; i < end; i += 32) a.y[i] = 0.f;
+        for (unsigned i = unsigned(r) + unsigned(lane); i < unsigned(end); i += 32) a.y[i] = 0.f;
         r = end;
         if (strides < 32 && stride == 32) break;
         stride = strides < 32 ? 32 : min(stride * 32, 1 << 25);

@@ -150,6 +150,9 @@ def skip_empty(rp, v, r, r1, cleared):
     while stride <= r1 - r:
         empty = [stride * (q + 1) <= r1 - r and rp[r + stride * (q + 1)] == v for q in range(32)]
         strides = sum(empty)
+        assert stride * 32 <= 2 ** 30 and r + stride * strides <= r1
+        # the clearing loop's index is unsigned: its last step may pass 2^31
+        assert r + stride * strides + 31 < 2 ** 32
         cleared.extend(range(r, r + stride * strides))
         r += stride * strides
         if strides < 32 and stride == 32:
@@ -175,3 +178,20 @@ def test_runs_of_empty_rows(run, after):
         r += 32
     assert cleared == list(range(r)) and r <= run
     assert run - r < 64
+
+
+class _Counted(list):
+    """Collects ranges without holding them."""
+
+    def __init__(self):
+        super().__init__()
+        self.rows = 0
+
+    def extend(self, rows):
+        self.rows += len(rows)
+
+
+def test_the_longest_run():
+    m = 2 ** 31 - 1
+    cleared = _Counted()
+    assert skip_empty(_Steps(m), 0, 0, m, cleared) == cleared.rows > m - 2 ** 25
