@@ -92,8 +92,16 @@ typedef struct pramaan_pdhg_options {
     int32_t algorithm;        /* PRAMAAN_ALGO_REFERENCE                        */
     int32_t termination;      /* PRAMAAN_TERM_REFERENCE                        */
     int32_t device;           /* CUDA device ordinal, default 0                */
-    int32_t use_graph;        /* 1: replay each check interval as a CUDA graph */
-    int32_t profile_kernels;  /* 1: time every product kernel with CUDA events */
+    int32_t use_graph;        /* 1: replay each check interval as a CUDA graph
+                                 (where the products run over tiles; an interval
+                                 that a cluster runs is one launch anyway)      */
+    int32_t profile_kernels;  /* 1: time every product kernel with CUDA events.
+                                 Reference algorithm: an LP whose iterations a
+                                 cluster would run from its shared memory (see
+                                 pramaan_session_path_info) then runs over tiles,
+                                 so the times are of kernels that a run without
+                                 this option launches only in calls of a few
+                                 iterations, and sums are added in another order */
     int32_t refine;           /* adaptive mode, 1 (default): FP64 master iterates
                                  on the device, the FP32 iteration runs on the
                                  correction and is folded into them at every
@@ -124,7 +132,9 @@ typedef struct pramaan_pdhg_options {
                                  faster (local column patterns); 1: as 0, but
                                  L1-cached gathers on every operand without hot
                                  entries; -1: plain L2 gathers only.  The
-                                 results are identical in every mode            */
+                                 results are identical in every mode; this and
+                                 launch_blocks concern products over tiles, not
+                                 LPs that run from a cluster's shared memory    */
     int32_t launch_blocks;    /* 0 (default): the launch autotuner picks the
                                  resident blocks per SM of the products over a
                                  large operand; > 0: that many (capped by what
@@ -425,7 +435,11 @@ PRAMAAN_API int pramaan_session_create(const pramaan_lp* lp, const pramaan_pdhg_
                            pramaan_pdhg_session** out);
 PRAMAAN_API int pramaan_session_destroy(pramaan_pdhg_session* s);
 /* Runs `iterations` PDHG iterations without convergence checks (asynchronous
- * on the session stream; graph replay when use_graph is set). */
+ * on the session stream; graph replay when use_graph is set).  An LP that fits
+ * a cluster's shared memory runs there in one launch from 2 + nnz / 15,000
+ * iterations on, and over tiles in shorter calls; the two add a row's products
+ * in different orders, so the last bits depend on how the iterations are cut
+ * into calls. */
 PRAMAAN_API int pramaan_session_iterate(pramaan_pdhg_session* s, int32_t iterations);
 /* Waits for the session stream. */
 PRAMAAN_API int pramaan_session_synchronize(pramaan_pdhg_session* s);

@@ -876,10 +876,11 @@ void AdaptiveBatch::launch_interval(int k) {
     }
 }
 
-// By default (persistent = 0) the cluster kernel takes the intervals once
-// the layout holds few enough LPs for clusters of kClusterAutoMin blocks (the
-// tail of a batch, or a single LP) and every LP has at most
-// kClusterAutoMaxNnz non-zeros; persistent = 2 takes it always.  Measured on
+// LPs that all fit a cluster's shared memory run from there (build_resident).
+// For the others the kernel that reads them from L2 takes the intervals by
+// default (persistent = 0) once the layout holds few enough LPs for clusters of
+// kClusterAutoMin blocks (the tail of a batch, or a single LP) and every LP has at
+// most kClusterAutoMaxNnz non-zeros; persistent = 2 takes it always.  Measured on
 // the rolling-horizon batch (128 LPs, T ~ U{24..336}, P ~ U{5..50}): its
 // slowest LP alone (66,704 non-zeros, 300 k iterations) at 10.1 us per
 // iteration against 17.9 on the tiled path; its first 16 and 32 LPs (clusters

@@ -219,13 +219,12 @@ struct SpmvSmemLayout {
 // In, value) declare `static constexpr bool kSplit = true`; the tile loop then
 // loads kEpiPass rows per lane ahead of their updates, and with `static
 // constexpr int kAhead` the first kAhead rows per lane while the tile's gathers
-// are in flight.  (All
-// warps of an SM gather and update at about the same time, so an update's
-// round trip leaves the gather path idle.)  us per reference iteration, no row
-// ahead | two: uniform 4 M non-zeros 51.5 | 49.0, banded 26 M 102.8 | 101.2;
-// with one row in the primal update, whose kernel spilled with two, 43.2 and 84.8
-// (row-aligned tiles, two in both 44.0 and 93.0).  The Halpern updates have more
-// inputs still: none ahead.
+// are in flight.  (All warps of an SM gather and update at about the same time,
+// so an update's round trip leaves the gather path idle.)  us per reference
+// iteration, no row ahead | two: uniform 4 M non-zeros 51.5 | 49.0, banded 26 M
+// 102.8 | 101.2; with one row in the primal update, whose kernel spilled with
+// two, 43.2 and 84.8 (row-aligned tiles, two in both 44.0 and 93.0).  The Halpern
+// updates have more inputs still: none ahead.
 template <class Epi, class = void>
 struct EpiSplit { static constexpr bool value = false; };
 template <class Epi>

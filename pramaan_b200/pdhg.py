@@ -125,8 +125,9 @@ class PdhgOptions:
     algorithm: int = 0          # 0: the reference iteration, 1: adaptive (PDLP-style), 2: Halpern
     termination: int | None = None  # default: reference criterion / relative KKT (adaptive)
     device: int = 0
-    use_graph: bool = True
-    profile_kernels: bool = False
+    use_graph: bool = True      # products over tiles: replay each check interval as a CUDA graph
+    profile_kernels: bool = False   # CUDA events around the products; small LPs of the reference
+                                # algorithm then run over tiles, not from a cluster's shared memory
     refine: bool = True         # adaptive mode: FP64 master iterates + FP32 corrections
     persistent: int = 0         # Halpern mode: 0 one cluster per LP runs each check interval, from its
                                 # shared memory when every LP fits, else from L2 for few LPs of
