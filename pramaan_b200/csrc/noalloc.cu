@@ -362,15 +362,15 @@ __device__ __forceinline__ void range_product(const NaArgs& a, const Words& word
             const int nd = __popc(__ballot_sync(0xffffffffu, done));
             // the next rows' pointers, before the sums of these
             int s2 = INT_MAX, s2_next = INT_MAX;
-            const int v = __shfl_sync(0xffffffffu, s, 0);
-            if (nd == 32 && s_next == v) {   // 32 empty rows: zeros, and on to the last row of the run
-                a.y[r + lane] = 0.f;
-                r = skip_empty(a, rp, v, r + 32, r1, lane);
-                s = lane <= r1 - r ? rp(r + lane) : INT_MAX;
-                s_next = 32 <= r1 - r ? rp(r + 32) : INT_MAX;
-                continue;
-            }
             if (nd == 32) {
+                const int v = __shfl_sync(0xffffffffu, s, 0);
+                if (s_next == v) {   // 32 empty rows: zeros, and on to the last row of the run
+                    a.y[r + lane] = 0.f;
+                    r = skip_empty(a, rp, v, r + 32, r1, lane);
+                    s = lane <= r1 - r ? rp(r + lane) : INT_MAX;
+                    s_next = 32 <= r1 - r ? rp(r + 32) : INT_MAX;
+                    continue;
+                }
                 s2 = 32 + lane <= r1 - r ? rp(r + 32 + lane) : INT_MAX;
                 s2_next = 64 <= r1 - r ? rp(r + 64) : INT_MAX;
             }
